@@ -210,6 +210,13 @@ struct HdgOps : LinearOps {
     else
       launch_block_inverse_apply(c, c.pc_hdg, c.nf, c.t, b, x);
   }
+  bool fused(const Ctx &c, int R) const override {
+    return c.opts.assembly != EG_ASSEMBLY_FULL && fused_solve_supported(c, R);
+  }
+  double solve_fused(Ctx &c, const KrylovBufs<double> &kb, const double *rhs, double *x, double tol, int limit,
+                     bool zero_guess, double rhs_norm, int *count) override {
+    return fused_solve_hdg(c, kb, rhs, x, tol, limit, zero_guess, rhs_norm, count);
+  }
 };
 
 static void pc_factor(Ctx &c, int form, bool factor) {
@@ -734,12 +741,7 @@ int eg_download(eg_ctx *ctx, int slot, double *dst) {
         }
       } else {
         if (!c.pc_hdg) eg::fail(EG_ERR_INVALID, "no preconditioner built");
-        if (!dst) eg::fail(EG_ERR_INVALID, "null vector");
-        // stored row-major for the block GEMV; the slot is column-major
-        eg::launch_transpose_blocks(c, c.pc_hdg, c.nf, c.t);
         eg::download_vec(c, dst, c.pc_hdg, (size_t)c.nf * c.t * c.t);
-        eg::launch_transpose_blocks(c, c.pc_hdg, c.nf, c.t);
-        c.sync();
       }
       return;
     }

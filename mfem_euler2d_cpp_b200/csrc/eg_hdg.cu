@@ -953,8 +953,7 @@ __global__ void __launch_bounds__(64)
       out = Inv;
     }
     for (int i = threadIdx.x; i < T; i += blockDim.x) pivots[(size_t)f * T + i] = factor ? piv_s[i] : i;
-    // stored row-major (one contiguous row per output of the block GEMV)
-    for (int o = threadIdx.x; o < T * T; o += blockDim.x) blocks[(size_t)f * T * T + (o % T) * T + o / T] = out[o];
+    for (int o = threadIdx.x; o < T * T; o += blockDim.x) blocks[(size_t)f * T * T + o] = out[o];
   }
 }
 
@@ -965,7 +964,7 @@ __global__ void __launch_bounds__(64)
 // Rows never move: the pivot row of step k ends up holding row k of S^{-1}.
 // The pivot search is three warp reductions on IEEE bit patterns and the
 // normalised pivot row is broadcast by shuffles, so no step needs a barrier.
-// `pivots` receives the pivot row of every step. Blocks are stored row-major.
+// `pivots` receives the pivot row of every step.
 template <int T>
 __global__ void __launch_bounds__(128)
     schur_jacobi_warp_kernel(int nx, int ny, int nf, int npan, const double *__restrict__ D,
@@ -990,11 +989,11 @@ __global__ void __launch_bounds__(128)
       sr[c] = row_ok ? ((lane == c ? d : 0.) - pl[c * T + lane]) - pr[c * T + lane] : 0.;
       xr[c] = lane == c ? 1. : 0.;
     }
-    double *out = blocks + (size_t)f * T * T;  // row-major
+    double *out = blocks + (size_t)f * T * T;  // column-major
     if (!factor) {
       if (row_ok) {
 #pragma unroll
-        for (int c = 0; c < T; ++c) out[lane * T + c] = sr[c];
+        for (int c = 0; c < T; ++c) out[c * T + lane] = sr[c];
         pivots[(size_t)f * T + lane] = lane;
       }
       continue;
@@ -1049,53 +1048,27 @@ __global__ void __launch_bounds__(128)
     }
     if (row_ok) {
 #pragma unroll
-      for (int c = 0; c < T; ++c) out[pos * T + c] = xr[c];
+      for (int c = 0; c < T; ++c) out[c * T + pos] = xr[c];
       pivots[(size_t)f * T + pos] = lane;
     }
   }
 }
 
-// x_b = Inv_b b_b for row-major bs x bs inverses (bs even); one thread per
-// output row, which reads its row with 16-byte loads. BS > 0 fixes the block
-// size at compile time, so the row loop unrolls and all of a row's loads are
-// in flight together (BS = 0: any even size).
+// x_b = Inv_b b_b for column-major BS x BS inverses: one thread per output
+// row, so that neighbouring threads read neighbouring entries of a column; the
+// column loop unrolls and all of a row's loads are in flight together.
 template <int BS>
-__global__ void __launch_bounds__(256) block_gemv_kernel(const double *__restrict__ inv, int nblocks, int bs_rt,
-                                                         const double *__restrict__ b,
-                                                         double *__restrict__ x, const int *__restrict__ skip) {
-  if (skip != nullptr && *skip) return;
-  const int bs = BS > 0 ? BS : bs_rt;
+__global__ void __launch_bounds__(256) block_gemv_kernel(const double *__restrict__ inv, int nblocks,
+                                                         const double *__restrict__ b, double *__restrict__ x) {
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= (long long)nblocks * bs) return;
-  const int blk = (int)(id / bs);
-  const double2 *ib = reinterpret_cast<const double2 *>(inv + (size_t)id * bs);
-  const double *bb = b + (size_t)blk * bs;
+  if (id >= (long long)nblocks * BS) return;
+  const int blk = (int)(id / BS), row = (int)(id % BS);
+  const double *a = inv + (size_t)blk * BS * BS + row;
+  const double *bb = b + (size_t)blk * BS;
   double acc = 0.;
 #pragma unroll
-  for (int c = 0; c < (BS > 0 ? BS / 2 : bs / 2); ++c) {
-    const double2 a = ib[c];
-    acc += a.x * bb[2 * c];
-    acc += a.y * bb[2 * c + 1];
-  }
+  for (int c = 0; c < BS; ++c) acc += a[c * BS] * bb[c];
   x[id] = acc;
-}
-
-// In-place transpose of every bs x bs block (one thread per pair i < j).
-__global__ void transpose_blocks_kernel(double *a, int nblocks, int bs) {
-  const long long per = (long long)bs * (bs - 1) / 2;
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= per * nblocks) return;
-  const int blk = (int)(id / per);
-  int k = (int)(id % per), i = 0;
-  while (k >= bs - 1 - i) {  // row i holds the pairs (i, i+1..bs-1)
-    k -= bs - 1 - i;
-    ++i;
-  }
-  const int j = i + 1 + k;
-  double *m = a + (size_t)blk * bs * bs;
-  const double t = m[i * bs + j];
-  m[i * bs + j] = m[j * bs + i];
-  m[j * bs + i] = t;
 }
 
 // ================================================================ launchers
@@ -1231,13 +1204,6 @@ void launch_recovered_residual(Ctx &c, const double *eq, double *er) {
   EG_CUDA(cudaGetLastError());
 }
 
-void launch_transpose_blocks(Ctx &c, double *a, int nblocks, int bs) {
-  const long long total = (long long)nblocks * bs * (bs - 1) / 2;
-  if (total == 0) return;
-  transpose_blocks_kernel<<<(unsigned)((total + 255) / 256), 256, 0, c.stream>>>(a, nblocks, bs);
-  EG_CUDA(cudaGetLastError());
-}
-
 void launch_block_inverse_apply(Ctx &c, const double *inv, int nblocks, int bs, const double *b, double *x) {
   ProfScope ps(c, EG_K_PC_APPLY, 1);
   const long long total = (long long)nblocks * bs;
@@ -1245,12 +1211,12 @@ void launch_block_inverse_apply(Ctx &c, const double *inv, int nblocks, int bs, 
   switch (bs) {
 #define EG_BG(BB)                                                                                  \
   case BB:                                                                                         \
-    block_gemv_kernel<BB><<<grid, 256, 0, c.stream>>>(inv, nblocks, bs, b, x, c.skip);             \
+    block_gemv_kernel<BB><<<grid, 256, 0, c.stream>>>(inv, nblocks, b, x);                         \
     break;
     EG_BG(4) EG_BG(8) EG_BG(12) EG_BG(16) EG_BG(20) EG_BG(24) EG_BG(28) EG_BG(32) EG_BG(36)
 #undef EG_BG
     default:
-      block_gemv_kernel<0><<<grid, 256, 0, c.stream>>>(inv, nblocks, bs, b, x, c.skip);
+      fail(EG_ERR_INVALID, "unsupported trace block size");
   }
   EG_CUDA(cudaGetLastError());
 }

@@ -87,6 +87,15 @@ struct ProfScope {
   ~ProfScope();
 };
 
+// Krylov workspace of one vector type: basis (R+1 columns, leading dimension
+// ld) and the work vectors of the solver.
+template <class T>
+struct KrylovBufs {
+  T *V, *w, *z, *res, *comb, *corr;
+  size_t ld;
+  int R;
+};
+
 // Operators used by the Krylov solver, on vectors of type T.
 template <class T>
 struct LinearOpsT {
@@ -98,6 +107,9 @@ struct LinearOpsT {
   int group = 1;
   virtual void apply(Ctx &c, const T *x, T *y) = 0;
   virtual void precondition(Ctx &c, const T *b, T *x) = 0;
+  // whether the whole solve runs as one launch (eg_gmres.cu), and that solve
+  virtual bool fused(const Ctx &, int) const { return false; }
+  virtual double solve_fused(Ctx &, const KrylovBufs<T> &, const T *, T *, double, int, bool, double, int *) { return 0.; }
   virtual ~LinearOpsT() = default;
 };
 using LinearOps = LinearOpsT<double>;
@@ -108,15 +120,6 @@ constexpr int kArnoldiGroup = 4;
 // Degrees whose Schur action streams the 16 panels C_s X_o of a cell (16 t^2
 // doubles) instead of X (m x 4t): fewer bytes from q = 5 (k = 4) on.
 __host__ __device__ constexpr bool schur_panels_full(int q) { return q >= 5; }
-
-// Krylov workspace of one vector type: basis (R+1 columns, leading dimension
-// ld) and the work vectors of the solver.
-template <class T>
-struct KrylovBufs {
-  T *V, *w, *z, *res, *comb, *corr;
-  size_t ld;
-  int R;
-};
 
 // Bound of a device-side wait of the block ILU(0) factor and sweeps. The
 // longest legitimate wait is bounded by one whole factor or sweep (45 ms for
@@ -214,6 +217,9 @@ struct Ctx {
          *kx = nullptr;
   GmresCtl *ctl = nullptr;
   GmresCtl *hctl = nullptr;  // pinned mirror
+  // one-launch GMRES (eg_gmres.cu): barrier words and published column sums
+  unsigned *solve_bar = nullptr;
+  double *solve_partials = nullptr;
   // set while GMRES enqueues a group of Arnoldi steps: the operator kernels
   // of those steps return at once when *skip (the device stop flag) is set
   const int *skip = nullptr;
@@ -298,10 +304,8 @@ void launch_schur_apply(Ctx &c, const double *v, double *y);
 void launch_recover(Ctx &c, const double *lam, double *du);
 void launch_recovered_residual(Ctx &c, const double *eq, double *er);
 void launch_schur_jacobi(Ctx &c, bool factor);
-// x = Inv b for explicit block inverses (Schur block Jacobi apply).
+// x = Inv b for explicit column-major block inverses (Schur block Jacobi apply).
 void launch_block_inverse_apply(Ctx &c, const double *inv, int nblocks, int bs, const double *b, double *x);
-// in-place transpose of every bs x bs block of `a`
-void launch_transpose_blocks(Ctx &c, double *a, int nblocks, int bs);
 // ---- eg_api.cu ----
 // Sets the context's description (geometry, tables, metrics) for its size.
 void upload_desc(Ctx &c, const eg_desc &d);
@@ -350,6 +354,14 @@ double gmres(Ctx &c, LinearOps &ops, const double *rhs, double *x, double tol, i
 // norm reached without requiring convergence (inner solve of mixed precision).
 double gmres_f32(Ctx &c, LinearOpsT<float> &ops, const KrylovBufs<float> &kb, const float *rhs, float *x,
                  double tol, int limit, int *count);
+// ---- one-launch GMRES with block Jacobi (eg_gmres.cu) ----
+bool fused_solve_supported(const Ctx &c, int R);
+// The iteration of gmres() for the condensed system, from a known rhs norm;
+// leaves rhs - A x in kb.res and returns its weighted norm.
+double fused_solve_hdg(Ctx &c, const KrylovBufs<double> &kb, const double *rhs, double *x, double tol, int limit,
+                       bool zero_guess, double rhs_norm, int *count);
+double fused_solve_hdg_f32(Ctx &c, const KrylovBufs<float> &kb, const float *rhs, float *x, double tol, int limit,
+                           double rhs_norm, int *count);
 // ---- eg_api.cu ----
 // One accepted damped Newton update (src/stepper.cpp:129-228).
 void newton_update(Ctx &c, double residual_norm, double old_norm, eg_update_stats *st);

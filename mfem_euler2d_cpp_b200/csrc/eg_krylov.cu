@@ -521,6 +521,14 @@ double gmres_t(Ctx &c, LinearOpsT<T> &ops, const KrylovBufs<T> &kb, const T *rhs
   const int R = std::min(N, kb.R);
   const size_t ldv = kb.ld;
   T *res = kb.res, *w = kb.w, *z = kb.z, *V = kb.V;
+  const double rhs_norm = known_rhs_norm >= 0. ? known_rhs_norm : wnorm_t(c, rhs, N, ops.mtab, ops.period);
+  if (rhs_norm_out) *rhs_norm_out = rhs_norm;
+  *count = 0;
+  if (rhs_norm != 0. && ops.fused(c, R)) {
+    const double res_norm = ops.solve_fused(c, kb, rhs, x, tol, limit, zero_guess, rhs_norm, count);
+    if (require_converged && !(res_norm <= tol * rhs_norm)) fail(EG_ERR_GMRES_LIMIT, "GMRES iteration limit reached");
+    return res_norm;
+  }
   if (zero_guess) {
     {
       ProfScope ps(c, EG_K_VECTOR, 1);
@@ -534,9 +542,6 @@ double gmres_t(Ctx &c, LinearOpsT<T> &ops, const KrylovBufs<T> &kb, const T *rhs
     sub_kernel<T><<<vec_grid(N), 256, 0, c.stream>>>(N, rhs, w, res);
     EG_CUDA(cudaGetLastError());
   }
-  const double rhs_norm = known_rhs_norm >= 0. ? known_rhs_norm : wnorm_t(c, rhs, N, ops.mtab, ops.period);
-  if (rhs_norm_out) *rhs_norm_out = rhs_norm;
-  *count = 0;
   if (rhs_norm == 0.) return 0.;
   int iterations = 0;
   // from a zero guess the residual is a copy of rhs: the same reduction result
