@@ -608,6 +608,23 @@ int sm_count_gmres() {
   return n;
 }
 
+// CTAs of a solve over `cells` cells whose operator streams `bytes` per step on
+// vectors of N entries: one per 256 KB or 444 entries, at least 16, at
+// most one per SM, and no CTA with a nearly idle second round of cells. More CTAs than that shorten a small solve by a few per cent and keep
+// other instances off the SMs: measured per step at 16x16 Q3 20.5, 17.5, 16.0,
+// 16.5 us with 16, 32, 64, 148 CTAs; 32x32 Q2 26.9, 19.7, 18.3 us with 32, 64,
+// 148; 64x64 Q1 34.9, 26.0 us with 64, 148; 20x20 Q8 37.2, 32.0, 30.6 us with
+// 64, 100, 148; a batch of six instances of 400 to 1024 cells takes 104 ms with
+// 148 CTAs each, 72 to 75 ms with 37 to 74.
+int solve_grid(int cells, double bytes, int N) {
+  const double want = std::max(16., std::max(bytes / 262144., N / 444.));
+  const int cap = std::min(sm_count_gmres(), cells);
+  const int grid = std::max(1, (int)std::min<double>(cap, std::ceil(want)));
+  int per = (cells + grid - 1) / grid;  // no more CTAs than the fullest ones need
+  if (per > kGW && per < 2 * kGW && (cells + kGW - 1) / kGW <= cap) per = kGW;
+  return (cells + per - 1) / per;
+}
+
 template <class Op>
 double launch_solve(Ctx &c, typename Op::Args &oa, SolveArgs<typename Op::Real> &s, int grid, int *count) {
   EG_CUDA(cudaMemsetAsync(s.bar.count, 0, sizeof(unsigned) + sizeof(int), c.stream));
@@ -656,13 +673,12 @@ template <int Q, class T, bool PAN>
 double solve_hdg(Ctx &c, const KrylovBufs<T> &kb, const T *act, const T *D, const T *pc, T *contrib, const T *rhs,
                  T *x, double tol, int limit, bool zero_guess, double rhs_norm, int *count) {
   using Op = HdgOp<Q, T, PAN>;
-  const int sms = sm_count_gmres();
-  const int grid = std::min(sms, c.n);
+  const size_t stride = PAN ? (size_t)16 * c.t * c.t
+                            : (sizeof(T) == 8 ? (size_t)c.m * (4 * c.t + 1) : (size_t)c.m * 4 * c.t);
+  const int grid = solve_grid(c.n, (double)c.n * Op::ROWS * Op::K * sizeof(T), c.nl);
   const int per = (c.n + grid - 1) / grid;
   int split = 1;
   while (split < kGW && 2 * split * per <= kGW) split *= 2;
-  const size_t stride = PAN ? (size_t)16 * c.t * c.t
-                            : (sizeof(T) == 8 ? (size_t)c.m * (4 * c.t + 1) : (size_t)c.m * 4 * c.t);
   typename Op::Args oa{c.geo, c.tab, c.Cb, act, stride, D, pc, contrib, split};
   SolveArgs<T> s = solve_args(c, kb, rhs, x, tol, limit, zero_guess, rhs_norm, c.nl);
   s.cells = c.n;
