@@ -112,8 +112,7 @@ void Ctx::prof_resolve() {
 }
 
 void Ctx::check_device_error() {
-  EG_CUDA(cudaMemcpyAsync(herr, derr, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  EG_CUDA(cudaMemcpyAsync(herr + 2, derr + 2, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  EG_CUDA(cudaMemcpyAsync(herr, derr, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream));
   sync();
   if (herr[2]) {
     broken = true;
@@ -134,6 +133,7 @@ void Ctx::ensure_hdg() {
   sf = alloc_n<double>((size_t)n * 4 * q);
   contrib = alloc_n<double>((size_t)n * 4 * t);
   panels = alloc_n<double>((size_t)n * geo.npan * t * t);
+  if (!redo) redo = alloc_n<int>(n);
   rhs = alloc_n<double>(nl);
   lam = alloc_n<double>(nl);
   tmp_trace = alloc_n<double>(nl);
@@ -345,8 +345,7 @@ void newton_update(Ctx &c, double residual_norm, double old_norm, eg_update_stat
     s.validation_s = now_s() - v0;
   } else {
     const double c0 = now_s();
-    launch_condense(c, c.u, c.r);
-    c.check_device_error();
+    condense(c, c.u, c.r);
     s.condensation_s = now_s() - c0;
     double tol = c.opts.linear_tol;
     bool valid = false;
@@ -836,8 +835,7 @@ int eg_condense(eg_ctx *ctx) {
   if (!ctx) return EG_ERR_INVALID;
   return guard(ctx, [&] {
     Ctx &c = ctx->c;
-    eg::launch_condense(c, c.u, c.r);
-    c.check_device_error();
+    eg::condense(c, c.u, c.r);
   });
 }
 

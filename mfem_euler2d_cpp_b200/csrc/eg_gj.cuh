@@ -3,20 +3,12 @@
 // the pivot reciprocal and the warp-level pivot selection of a 4-column
 // panel. Not part of the public C-ABI.
 #pragma once
+#include "eg_cellinv.cuh"
 #include "eg_device.cuh"
 
 namespace eg {
 
 // ------------------------------------------- tensor-core Gauss-Jordan
-// D = C + A B on the FP64 tensor pipe: m8n8k4, A row-major 8x4 (one element
-// per lane: row lane/4, column lane%4), B column-major 4x8 (row lane%4,
-// column lane/4), C/D 8x8 (two elements per lane: row lane/4, columns
-// 2*(lane%4) and 2*(lane%4)+1).
-__device__ __forceinline__ void dmma_m8n8k4(double &d0, double &d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
 
 // Reciprocal of a pivot: hardware estimate refined by two Newton-Raphson
 // steps r <- r + r (1 - x r) (quadratic convergence from the ~2^-20 estimate;

@@ -10,6 +10,7 @@
 //              deterministic).
 #include <algorithm>
 
+#include "eg_cellinv.cuh"
 #include "eg_cellmat.cuh"
 #include "eg_gj.cuh"
 #include "eg_internal.h"
@@ -170,84 +171,21 @@ __device__ void condense_epilogue(const CondenseShared<Q> &sh, const double *R, 
   }
 }
 
-// Entry (row, col) of the lift B (col < 4t) of the cell system: the face
-// point's scalar lift sf times phi * inv_mass on the component of the column
-// (HybridCell's B, src/problem.cpp:622-630; the same values condense_build
-// writes). SF is the cell's staged lift scalars.
-template <int Q>
-__device__ __forceinline__ double lift_entry(const STab<Q> &st, const double *SF, int row, int col) {
-  constexpr int T = 4 * Q;
-  const int s = col / T, rem = col % T, jj = rem >> 2, c = rem & 3;
-  const int i = row >> 2;
-  if ((row & 3) != c) return 0.;
-  const int ix = i % Q, iy = i / Q;
-  const bool on = s < 2 ? iy == jj : ix == jj;
-  if (!on) return 0.;
-  const int l = s < 2 ? ix : iy;
-  return st.fb(s, jj, l) * st.inv_mass(i) * SF[s * Q + jj];
-}
-
-// Outputs of a solved cell from R = [X | y] (stride ldr, unknown order):
-// [X | y] to XY (compact), the trace contributions C_e y_e and the Schur
-// panels C_s X_o (src/condensation.cpp:141-142, src/operators.cpp:7-26). One
-// thread per (side, column) forms the column's trace on the side once
-// (q face points x 4 components) and applies the side's 4x4 flux blocks,
-// emitting 4q consecutive outputs.
-template <int Q>
-__device__ void condense_epilogue_traces(const CondenseShared<Q> &sh, const double *R, int ldr, double *XY,
-                                         double *contrib, double *panels, int npan, int e) {
-  constexpr int P = Q * Q, M = 4 * P, T = 4 * Q, NR = 4 * T + 1;
-  const STab<Q> &st = sh.st;
-  double *dst = XY + (size_t)e * M * NR;
-  for (int i = threadIdx.x; i < M * NR; i += blockDim.x) dst[i] = R[(size_t)(i / M) * ldr + i % M];
-  const bool all16 = npan == 16;
-  for (int task = threadIdx.x; task < 4 * NR; task += blockDim.x) {
-    const int s = task & 3, col = task >> 2;
-    const int so = col / T;  // block column of X (4 = y)
-    if (col < 4 * T && !all16 && so != s) continue;
-    double *out;
-    if (col == 4 * T) {
-      out = contrib + (size_t)e * 4 * T + s * T;
-    } else {
-      if (panels == nullptr) continue;
-      const int pan = all16 ? s * 4 + so : s;
-      out = panels + (((size_t)e * npan + pan) * T + (col - so * T)) * T;
-    }
-    const double *xc = R + (size_t)col * ldr;
-    for (int jj = 0; jj < Q; ++jj) {
-      double v[4] = {0., 0., 0., 0.};
-#pragma unroll
-      for (int l = 0; l < Q; ++l) {
-        const double f = st.fb(s, jj, l);
-        const double *xv = xc + 4 * line_node<Q>(s, jj, l);
-#pragma unroll
-        for (int d = 0; d < 4; ++d) v[d] += f * xv[d];
-      }
-      const double *cb = sh.CB + (s * Q + jj) * 16;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        double res = 0.;
-#pragma unroll
-        for (int d = 0; d < 4; ++d) res += cb[c + 4 * d] * v[d];
-        out[jj * 4 + c] = res;
-      }
-    }
-  }
-}
-
 // Generic condensation (any degree): CTA-cooperative LU on shared or global
 // memory (StreamCondense, src/condensation.cpp:131-148).
 template <int Q>
 __global__ void __launch_bounds__(256)
     condense_kernel(Geo g, const double *__restrict__ tab, Frozen fz, const double *__restrict__ u,
                     const double *__restrict__ r, double *XY, double *Cb, double *sf_out,
-                    double *contrib, double *panels, double *work, int *err) {
+                    double *contrib, double *panels, double *work, const int *__restrict__ list, int count,
+                    int *err) {
   constexpr int P = Q * Q, M = 4 * P, T = 4 * Q, NR = 4 * T + 1;
   constexpr int MODE = condense_mode<Q>();
   __shared__ CondenseShared<Q> sh;
   extern __shared__ double dyn[];
   load_tables<Q>(sh.st, tab);
-  for (int e = blockIdx.x; e < g.n; e += gridDim.x) {
+  for (int item = blockIdx.x; item < count; item += gridDim.x) {
+    const int e = list[item];
     __syncthreads();
     double *A = MODE < 2 ? dyn : work + (size_t)blockIdx.x * M * M;
     double *R = MODE == 0 ? dyn + (size_t)M * M : XY + (size_t)e * M * NR;
@@ -259,285 +197,6 @@ __global__ void __launch_bounds__(256)
       continue;
     }
     condense_epilogue<Q>(sh, R, MODE == 0, XY, contrib, panels, g.npan, e);
-  }
-}
-
-template <int Q, int WR, int WC>
-struct GjCfg {
-  static constexpr int P = Q * Q, M = 4 * P, T = 4 * Q, NR = 4 * T + 1, NC = M + NR;
-  static constexpr int MT = (M + 7) / 8, NT = (NC + 7) / 8;
-  static constexpr int TRW = (MT + WR - 1) / WR, TCW = (NT + WC - 1) / WC;
-  static constexpr int MP = 8 * TRW * WR, NP = 8 * TCW * WC;  // padded to whole warp tile grids
-  static constexpr int THREADS = 32 * WR * WC;
-  static constexpr int LD = M + 1;           // odd staging stride: conflict-free columns
-  static constexpr int KR = (M + 31) / 32;   // rows per lane in the pivot search
-};
-
-
-// Blocked Gauss-Jordan condensation on the tensor cores. The augmented cell
-// system W = [A | B | r_e] lives in registers as 8x8 accumulator tiles; warp
-// (wr, wc) owns tiles (wr + a*WR, wc + b*WC) of a tile grid padded with zero
-// rows and columns to whole warp grids. Panels are 4 columns wide:
-//  * the 4 pivot rows of panel p publish their trailing columns W_top;
-//  * one m8n8k4 MMA per trailing tile applies W_i -= A_i T^{-1} W_top with
-//    the A operand A_i = W_i[panel] for ordinary rows and A_i = T_r - e_r for
-//    pivot row r, which turns the same MMA into the row normalisation
-//    W_r -> (T^{-1} W_top)_r; B fragments T^{-1} W_top are formed per lane;
-//  * the tile column holding panel p+1 (always the first trailing one) is
-//    staged right after its MMAs, and warp 0 selects the pivots of panel
-//    p+1 while the tensor pipe drains the rest of panel p.
-// Pivot selection is partial pivoting over the rows not yet used: largest
-// magnitude after eliminating the panel's earlier pivots with multipliers
-// a_ij * (1/pivot), first row on ties (MFEM LUFactors::Factor), found with
-// warp max/min reductions on the IEEE bit pattern. Pivoting is virtual (rows
-// never move): after the last panel, row pivrow[j] holds unknown j, so the
-// right-hand-side columns hold X_e = A_e^{-1} B_e and y_e = A_e^{-1} r_e,
-// permuted back on the way out (StreamCondense, src/condensation.cpp:136-140,
-// carried to reduced row echelon form: no triangular solve follows).
-template <int Q, int WR, int WC, int MINB>
-__global__ void __launch_bounds__(32 * WR *WC, MINB)
-    condense_gj_kernel(Geo g, const double *__restrict__ tab, Frozen fz, const double *__restrict__ u,
-                       const double *__restrict__ r, double *XY, double *Cb, double *sf_out,
-                       double *contrib, double *panels, int *err) {
-  using C = GjCfg<Q, WR, WC>;
-  constexpr int M = C::M, NC = C::NC, MP = C::MP, NP = C::NP;
-  constexpr int TRW = C::TRW, TCW = C::TCW, LD = C::LD, KR = C::KR, NPAN = M / 4;
-  __shared__ CondenseShared<Q> sh;
-  __shared__ double pan[2][MP][4], top[2][4][NP];
-  __shared__ double fac[2][16];   // T^{-1} of the panel's pivot block, row-major 4x4
-  __shared__ int pivs[2][4];
-  __shared__ int invp[MP];
-  __shared__ unsigned char used[MP];
-  __shared__ int sing;
-  extern __shared__ double dyn[];  // staged system, column-major M x NC, stride LD
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wr = warp % WR, wc = warp / WR;
-  const int gq = lane >> 2, tq = lane & 3;
-  load_tables<Q>(sh.st, tab);
-
-  // Warp 0: choose the 4 pivots of the panel staged in pan[buf]; publish
-  // T^{-1} and turn the pivot rows of the A operand into T_r - e_r.
-  auto select = [&](int jbase, int buf) {
-    return gj_select_pivots<M, KR>(jbase, pan[buf], fac[buf], pivs[buf], used, invp, lane);
-  };
-
-  for (int e = blockIdx.x; e < g.n; e += gridDim.x) {
-    __syncthreads();
-    condense_build<Q>(sh, g, fz, u, r, Cb, sf_out, dyn, dyn + (size_t)LD * M, e, LD);
-    for (int i = threadIdx.x; i < MP; i += C::THREADS) {
-      used[i] = i >= M ? 1 : 0;
-      invp[i] = 0;
-    }
-    if (threadIdx.x == 0) sing = 0;
-    __syncthreads();
-    double acc[TRW][TCW][2];
-#pragma unroll
-    for (int a = 0; a < TRW; ++a) {
-      const int row = (wr + a * WR) * 8 + gq;
-#pragma unroll
-      for (int b = 0; b < TCW; ++b) {
-        const int col = (wc + b * WC) * 8 + 2 * tq;
-        acc[a][b][0] = (row < M && col < NC) ? dyn[row + (size_t)col * LD] : 0.;
-        acc[a][b][1] = (row < M && col + 1 < NC) ? dyn[row + (size_t)(col + 1) * LD] : 0.;
-      }
-    }
-    // stage panel 0 (tile column 0, left half)
-    if (wc == 0 && tq < 2) {
-#pragma unroll
-      for (int a = 0; a < TRW; ++a) {
-        const int row = (wr + a * WR) * 8 + gq;
-        pan[0][row][2 * tq] = acc[a][0][0];
-        pan[0][row][2 * tq + 1] = acc[a][0][1];
-      }
-    }
-    __syncthreads();
-    if (warp == 0 && !select(0, 0) && lane == 0) sing = 1;
-    __syncthreads();
-#pragma unroll 1
-    for (int p = 0; p < NPAN && !sing; ++p) {
-      const int j = 4 * p, pb = p & 1;
-      const int pr0 = pivs[pb][0], pr1 = pivs[pb][1], pr2 = pivs[pb][2], pr3 = pivs[pb][3];
-      const int tstart = (j + 4) >> 3;  // first tile column holding columns >= j+4 (= panel p+1's)
-      // publish the trailing columns of the pivot rows (zero left of j+4)
-#pragma unroll
-      for (int a = 0; a < TRW; ++a) {
-        const int row = (wr + a * WR) * 8 + gq;
-        const int rr = row == pr0 ? 0 : row == pr1 ? 1 : row == pr2 ? 2 : row == pr3 ? 3 : -1;
-        if (rr >= 0) {
-#pragma unroll
-          for (int b = 0; b < TCW; ++b) {
-            const int tj = wc + b * WC;
-            if (tj >= tstart) {
-              const int col = tj * 8 + 2 * tq;
-              top[pb][rr][col] = col >= j + 4 ? acc[a][b][0] : 0.;
-              top[pb][rr][col + 1] = col + 1 >= j + 4 ? acc[a][b][1] : 0.;
-            }
-          }
-        }
-      }
-      __syncthreads();
-      // A operands (row gq, column tq of each tile row) and B operands
-      // (row tq, column gq of each tile column) = T^{-1} top
-      double af[TRW];
-#pragma unroll
-      for (int a = 0; a < TRW; ++a) af[a] = -pan[pb][(wr + a * WR) * 8 + gq][tq];
-      const double *F = fac[pb];
-      const double f0 = F[4 * tq], f1 = F[4 * tq + 1], f2 = F[4 * tq + 2], f3 = F[4 * tq + 3];
-      const bool more = p + 1 < NPAN;
-      const int jn = j + 4, half = (jn >> 2) & 1, nb = pb ^ 1;
-      const bool stager = more && wc == tstart % WC && (tq >> 1) == half;
-#pragma unroll
-      for (int b = 0; b < TCW; ++b) {
-        const int tj = wc + b * WC;
-        if (tj >= tstart) {
-          const int col = tj * 8 + gq;
-          const double bf = f0 * top[pb][0][col] + f1 * top[pb][1][col] + f2 * top[pb][2][col] +
-                            f3 * top[pb][3][col];
-#pragma unroll
-          for (int a = 0; a < TRW; ++a) dmma_m8n8k4(acc[a][b][0], acc[a][b][1], af[a], bf);
-          if (tj == tstart && stager) {
-#pragma unroll
-            for (int a = 0; a < TRW; ++a) {
-              const int row = (wr + a * WR) * 8 + gq;
-              pan[nb][row][2 * (tq & 1)] = acc[a][b][0];
-              pan[nb][row][2 * (tq & 1) + 1] = acc[a][b][1];
-            }
-          }
-        }
-      }
-      __syncthreads();
-      if (more && warp == 0 && !select(jn, nb) && lane == 0) sing = 1;
-      __syncthreads();
-    }
-    if (sing) {
-      if (threadIdx.x == 0) raise_err(err, DERR_SINGULAR_CELL);
-      continue;
-    }
-    // right-hand sides back to unknown order: R(invp[w], col) = W(w, M + col)
-    double *R = dyn;  // compact M x NR, stride M (the staged system is no longer needed)
-#pragma unroll
-    for (int a = 0; a < TRW; ++a) {
-      const int row = (wr + a * WR) * 8 + gq;
-      if (row < M) {
-        const int jrow = invp[row];
-#pragma unroll
-        for (int b = 0; b < TCW; ++b) {
-          const int col = (wc + b * WC) * 8 + 2 * tq;
-          if (col >= M && col < NC) R[(size_t)(col - M) * M + jrow] = acc[a][b][0];
-          if (col + 1 >= M && col + 1 < NC) R[(size_t)(col + 1 - M) * M + jrow] = acc[a][b][1];
-        }
-      }
-    }
-    __syncthreads();
-    condense_epilogue<Q>(sh, R, true, XY, contrib, panels, g.npan, e);
-  }
-}
-
-// ------------------------------------- two-phase condensation (k = 3..5)
-// The cell system [A | B | r_e] of the register-resident kernel above fills
-// an SM's register file, so one cell's serial pivot chain leaves the SM idle
-// most of the time. This kernel splits the elimination so that two or three
-// cells share an SM at k = 3, 4 (CTAs of 8 warps, at most 128 registers per
-// thread, one copy of A per CTA in shared memory); at k = 5 A takes 164 KB
-// and one CTA of 16 warps fills the SM:
-//  1. Gauss-Jordan on A alone, in shared memory, in 4-column panels: warp 0
-//     picks the panel's pivots (gj_pick_pivots) and forms T^{-1}
-//     (gj_pivot_block_inverse) while the other warps copy the pivot rows'
-//     trailing columns; then every warp updates its trailing 8x8 tiles of A
-//     with one m8n8k4 FP64 MMA each (W_i -= a_i T^{-1} W_top, a_i = T_r - e_r
-//     on pivot rows), loads first, then MMAs, then stores. The panel columns
-//     are never touched again: together with T^{-1} and the pivot rows they
-//     are the record of the elimination.
-//  2. The record is replayed on [B | r_e] held in registers as 8x8 tiles
-//     (staged through the cell's own slot of XY, which the epilogue then
-//     overwrites with [X | y]): per panel the pivot rows are published and
-//     one MMA per tile applies the same update. No search runs in this phase.
-// The arithmetic is the register kernel's (the same pivots up to ties
-// within 2^-13, 2^-12 at k = 5, the same panel updates), so the results agree with the
-// reference's LU solve (src/condensation.cpp:131-148) to rounding.
-template <int Q, int MINB, int WR_ = 2, int WC_ = 4>
-__global__ void __launch_bounds__(32 * WR_ *WC_, MINB)
-    condense_gj2_kernel(Geo g, const double *__restrict__ tab, Frozen fz, const double *__restrict__ u,
-                        const double *__restrict__ r, double *XY, double *Cb, double *sf_out, double *contrib,
-                        double *panels, int *err) {
-  using C = Gj2Cfg<4 * Q * Q, 16 * Q + 1, WR_, WC_>;
-  constexpr int M = C::M, NR = C::NR, WR = C::WR, WC = C::WC;
-  constexpr int TRW = C::TRW, TCW = C::TCW, NPAN = C::NPAN, KR = C::KR;
-  constexpr int NP = C::NP, NQ = C::NQ, LDA = C::LDA;
-  __shared__ CondenseShared<Q> sh;
-  __shared__ double topA[4][NP];      // pivot rows of A (trailing columns) for the phase-1 update
-  __shared__ double topR[2][4][NQ];   // pivot rows of [B | r_e] in phase 2 (double-buffered)
-  __shared__ double rowbuf[KR * 32][4];
-  __shared__ double fac[NPAN][16];    // T^{-1} of every panel (row-major 4x4)
-  __shared__ int pivs[NPAN][4];
-  __shared__ int invp[KR * 32];
-  __shared__ unsigned char used[KR * 32];
-  __shared__ int sing;
-  extern __shared__ __align__(16) double A[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wr = warp % WR, wc = warp / WR;
-  const int gq = lane >> 2, tq = lane & 3;
-  load_tables<Q>(sh.st, tab);
-  for (int e = blockIdx.x; e < g.n; e += gridDim.x) {
-    __syncthreads();
-    condense_build<Q>(sh, g, fz, u, r, Cb, sf_out, A, nullptr, e, LDA);
-    // [B | r_e] is staged in the cell's slot of XY (L2-resident until
-    // [X | y] overwrites it), one element per thread in address order, by
-    // the warps that wait while warp 0 searches each panel's pivots: panel p
-    // stages the p-th of NPAN slices
-    double *Rg = XY + (size_t)e * M * NR;
-    const double *re = r + (size_t)e * M;
-    const auto stage = [&](int p, int t, int nt) {
-      constexpr int SL = (M * NR + NPAN - 1) / NPAN;
-      const int end = min(M * NR, (p + 1) * SL);
-      for (int i = p * SL + t; i < end; i += nt) {
-        const int col = i / M, row = i % M;
-        Rg[i] = col == NR - 1 ? re[row] : lift_entry<Q>(sh.st, sh.SF, row, col);
-      }
-    };
-    for (int i = threadIdx.x; i < KR * 32; i += C::THREADS) {
-      used[i] = i >= M ? 1 : 0;
-      invp[i] = 0;
-    }
-    if (threadIdx.x == 0) sing = 0;
-    __syncthreads();
-    // ------------------------------------------------ phase 1: reduce A
-    gj2_reduce<C>(A, topA, rowbuf, fac, pivs, used, invp, &sing, stage);
-    // ----------------------------- phase 2: replay on [B | r_e] (registers)
-    double acc[TRW][TCW][2];
-#pragma unroll
-    for (int a = 0; a < TRW; ++a) {
-      const int row = (wr + a * WR) * 8 + gq;
-#pragma unroll
-      for (int b = 0; b < TCW; ++b) {
-        const int col = (wc + b * WC) * 8 + 2 * tq;
-        acc[a][b][0] = (row < M && col < NR) ? Rg[row + (size_t)col * M] : 0.;
-        acc[a][b][1] = (row < M && col + 1 < NR) ? Rg[row + (size_t)(col + 1) * M] : 0.;
-      }
-    }
-    gj2_replay<C, TCW>(A, fac, pivs, topR, acc);
-    __syncthreads();  // the record in A is no longer read
-    if (sing) {
-      if (threadIdx.x == 0) raise_err(err, DERR_SINGULAR_CELL);
-      continue;
-    }
-    // right-hand sides back to unknown order: R(invp[w], col) = W(w, col)
-    double *R = A;  // M x NR, odd stride M + 1 (conflict-free column reads in the epilogue)
-#pragma unroll
-    for (int a = 0; a < TRW; ++a) {
-      const int row = (wr + a * WR) * 8 + gq;
-      if (row < M) {
-        const int jrow = invp[row];
-#pragma unroll
-        for (int b = 0; b < TCW; ++b) {
-          const int col = (wc + b * WC) * 8 + 2 * tq;
-          if (col < NR) R[(size_t)col * (M + 1) + jrow] = acc[a][b][0];
-          if (col + 1 < NR) R[(size_t)(col + 1) * (M + 1) + jrow] = acc[a][b][1];
-        }
-      }
-    }
-    __syncthreads();
-    condense_epilogue_traces<Q>(sh, R, M + 1, XY, contrib, panels, g.npan, e);
   }
 }
 
@@ -785,6 +444,189 @@ __global__ void __launch_bounds__(256, GjgCfg<Q>::MINB)
     }
     __syncthreads();
     condense_epilogue<Q>(sh, R, false, XY, contrib, panels, g.npan, e);
+  }
+}
+
+// --------------------------------------- condensation (k <= 5): cell inverses
+// Per cell: A is assembled in shared memory, inverted in registers by the
+// block Gauss-Jordan of eg_cellinv.cuh, and written back; X = A^{-1} B, y and
+// the panels follow from the inverse, since a column of B has q entries (the
+// nodes of one line, weighted by `lift`). For m <= 144 that takes fewer flops
+// than eliminating the 4t + 1 right-hand sides (2 m^3 against m^3 + 2 m^2
+// (4t + 1): 2.0 against 2.6 M at k = 4), needs no registers for them, and the
+// matrix fits an SM twice at k = 4.
+template <int Q>
+struct CondenseInvShared {
+  static constexpr int M = 4 * Q * Q;
+  STab<Q> st;
+  alignas(16) double us[M], rs[M], y[M], UT[16 * Q], FM[64 * Q], CB[64 * Q], SF[4 * Q], lift[4 * Q * Q];
+  int bad;
+};
+
+// Traces, face matrices FM = sign J(U_own) + stab I (stab = a or b), flux
+// blocks C = -ew FM and lift scalars B = -dt len/|K| ew stab of a cell
+// (src/problem.cpp:622-630, 661-699); the node Jacobians go to J.
+template <int Q>
+__device__ __forceinline__ void condense_cell_data(CondenseInvShared<Q> &sh, const Geo &g, const Frozen &fz,
+                                                   const double *__restrict__ u, const double *__restrict__ r, double *Cb,
+                                                   double *sf_out, double *J, int e) {
+  constexpr int M = 4 * Q * Q;
+  for (int i = threadIdx.x; i < M; i += blockDim.x) {
+    sh.us[i] = u[(size_t)e * M + i];
+    sh.rs[i] = r[(size_t)e * M + i];
+  }
+  if (threadIdx.x == 0) sh.bad = 0;
+  __syncthreads();
+  cell_traces<Q>(sh.st, sh.us, sh.UT);
+  node_jacobians<Q>(J, sh.st, sh.us, g);
+  __syncthreads();
+  for (int task = threadIdx.x; task < 4 * Q; task += blockDim.x) {
+    const int s = task / Q, j = task % Q;
+    const bool L = side_is_left(s);
+    const int fi = cell_face(e, s, g.nx, g.ny) * Q + j;
+    const double stab = L ? fz.a[fi] : fz.b[fi], ewj = sh.st.ew(j), nsign = L ? 1. : -1.;
+    double jm[16];
+    jacobian_axis(sh.UT + 4 * task, s >> 1, g.gm1, jm);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const double v = nsign * jm[k] + ((k % 5) == 0 ? stab : 0.);
+      sh.FM[task * 16 + k] = v;
+      sh.CB[task * 16 + k] = -ewj * v;
+    }
+    const double sv = -(g.dt * (s < 2 ? g.hy : g.hx) / g.area * ewj) * stab;
+    sh.SF[task] = sv;
+    sf_out[(size_t)e * 4 * Q + task] = sv;
+    for (int l = 0; l < Q; ++l) {
+      const int i = line_node<Q>(s, j, l);
+      sh.lift[task * Q + l] = sh.st.fb(s, j, l) * sh.st.inv_mass(i) * sv;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 64 * Q; i += blockDim.x) Cb[(size_t)e * 64 * Q + i] = sh.CB[i];
+}
+
+// Row r of V B for the four sides, from a matrix V whose column c starts at V
+// + c * ld: entry jc = 4 jj + c of every side is a weighted sum over the
+// x-line (sides 0, 1) or the y-line (sides 2, 3) through face point jj.
+template <int Q>
+__device__ __forceinline__ void lift_row(const double *lift, const double *V, int ld, int jc, double (&x)[4]) {
+  const int jj = jc >> 2, c = jc & 3;
+  x[0] = x[1] = x[2] = x[3] = 0.;
+#pragma unroll
+  for (int l = 0; l < Q; ++l) {
+    const double vx = V[(size_t)(4 * (jj * Q + l) + c) * ld], vy = V[(size_t)(4 * (l * Q + jj) + c) * ld];
+    x[0] += lift[jj * Q + l] * vx;
+    x[1] += lift[(Q + jj) * Q + l] * vx;
+    x[2] += lift[(2 * Q + jj) * Q + l] * vy;
+    x[3] += lift[(3 * Q + jj) * Q + l] * vy;
+  }
+}
+
+template <int Q, int WR, int WC>
+__host__ __device__ constexpr int condense_inv_aux() {  // doubles of J, later of one side's C R A^{-1}
+  constexpr int P = Q * Q, M = 4 * P, T = 4 * Q;
+  return 32 * P > M * T ? 32 * P : M * T;
+}
+
+template <int Q, int WR, int WC, int MINB>
+__global__ void __launch_bounds__(32 * WR *WC, MINB)
+    condense_inv_kernel(Geo g, const double *__restrict__ tab, Frozen fz, const double *__restrict__ u,
+                        const double *__restrict__ r, double *XY, double *Cb, double *sf_out, double *contrib,
+                        double *panels, int *redo, int *redo_count) {
+  using C = InvCfg<Q, WR, WC>;
+  constexpr int M = C::M, T = C::T, NR = 4 * T + 1, LDA = C::LDA;
+  __shared__ CondenseInvShared<Q> sh;
+  __shared__ __align__(16) double tiles[256];
+  extern __shared__ __align__(16) double A[];
+  double *aux = A + C::REGION;
+  load_tables<Q>(sh.st, tab);
+  for (int e = blockIdx.x; e < g.n; e += gridDim.x) {
+    __syncthreads();
+    condense_cell_data<Q>(sh, g, fz, u, r, Cb, sf_out, aux, e);
+    assemble_cell<C, Q>(A, sh.st, aux, sh.FM, g);
+    __syncthreads();
+    double acc[C::TR][C::TC][2];
+    load_tiles<C>(acc, A);
+    __syncthreads();  // the panels take the matrix's place
+    invert_tiles<C>(acc, A, tiles, &sh.bad);
+    if (sh.bad) {
+      if (threadIdx.x == 0) redo[atomicAdd(redo_count, 1)] = e;
+      continue;
+    }
+    store_tiles<C>(acc, A);
+    __syncthreads();
+    double *X = XY + (size_t)e * M * NR;
+    for (int t = threadIdx.x; t < M * T; t += blockDim.x) {
+      const int row = t % M, jc = t / M;
+      double x[4];
+      lift_row<Q>(sh.lift, A + row, LDA, jc, x);
+#pragma unroll
+      for (int s = 0; s < 4; ++s) X[(size_t)(s * T + jc) * M + row] = x[s];
+    }
+    for (int row = threadIdx.x; row < M; row += blockDim.x) {
+      double y[4] = {0., 0., 0., 0.};
+#pragma unroll 4
+      for (int c = 0; c < M; c += 4)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] += A[row + (size_t)(c + k) * LDA] * sh.rs[c + k];
+      const double v = (y[0] + y[1]) + (y[2] + y[3]);
+      sh.y[row] = v;
+      X[(size_t)(4 * T) * M + row] = v;
+    }
+    // one side at a time: C_s R_s A^{-1} (t x m, in aux), then its panels
+    for (int s = 0; s < 4; ++s) {
+      __syncthreads();
+      for (int t = threadIdx.x; t < Q * M; t += blockDim.x) {
+        const int jj = t / M, col = t % M;
+        double v[4] = {0., 0., 0., 0.};
+#pragma unroll
+        for (int l = 0; l < Q; ++l) {
+          const double f = sh.st.fb(s, jj, l);
+          const double2 *p = reinterpret_cast<const double2 *>(A + (size_t)col * LDA + 4 * line_node<Q>(s, jj, l));
+          const double2 p0 = p[0], p1 = p[1];
+          v[0] += f * p0.x;
+          v[1] += f * p0.y;
+          v[2] += f * p1.x;
+          v[3] += f * p1.y;
+        }
+        const double *cb = sh.CB + (s * Q + jj) * 16;
+        double o[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) o[c] = (cb[c] * v[0] + cb[c + 4] * v[1]) + (cb[c + 8] * v[2] + cb[c + 12] * v[3]);
+        double2 *dst = reinterpret_cast<double2 *>(aux + (size_t)col * T + 4 * jj);
+        dst[0] = make_double2(o[0], o[1]);
+        dst[1] = make_double2(o[2], o[3]);
+      }
+      if (s == 0) {
+        // C_s R_s y of every side (src/condensation.cpp:141-142)
+        for (int t = threadIdx.x; t < 4 * Q; t += blockDim.x) {
+          double v[4] = {0., 0., 0., 0.};
+          for (int l = 0; l < Q; ++l) {
+            const double f = sh.st.fb(t / Q, t % Q, l);
+            const double *p = sh.y + 4 * line_node<Q>(t / Q, t % Q, l);
+#pragma unroll
+            for (int d = 0; d < 4; ++d) v[d] += f * p[d];
+          }
+          const double *cb = sh.CB + t * 16;
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            contrib[(size_t)e * 4 * T + 4 * t + c] =
+                (cb[c] * v[0] + cb[c + 4] * v[1]) + (cb[c + 8] * v[2] + cb[c + 12] * v[3]);
+        }
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < T * T; t += blockDim.x) {
+        const int row = t % T, jc = t / T;
+        double x[4];
+        lift_row<Q>(sh.lift, aux + row, T, jc, x);
+        if (g.npan == 16) {
+#pragma unroll
+          for (int o = 0; o < 4; ++o) panels[(((size_t)e * 16 + s * 4 + o) * T + jc) * T + row] = x[o];
+        } else {
+          panels[(((size_t)e * 4 + s) * T + jc) * T + row] = x[s];
+        }
+      }
+    }
   }
 }
 
@@ -1083,30 +925,6 @@ static int sm_count_hdg() {
   return n;
 }
 
-static int condense_grid(Ctx &c) { return std::min(c.n, sm_count_hdg() * 4); }
-
-template <int Q, int WR, int WC, int MINB>
-static void launch_condense_gj(Ctx &c, const double *u, const double *r) {
-  using C = GjCfg<Q, WR, WC>;
-  constexpr size_t dyn = sizeof(double) * (size_t)C::LD * C::NC;
-  auto kern = condense_gj_kernel<Q, WR, WC, MINB>;
-  if (dyn > 48 * 1024)
-    EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-  const int grid = std::min(c.n, sm_count_hdg() * MINB);
-  kern<<<grid, C::THREADS, dyn, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, r,
-                                            c.XY, c.Cb, c.sf, c.contrib, c.panels, c.derr);
-}
-
-template <int Q, int MINB, int WR = 2, int WC = 4>
-static void launch_condense_gj2(Ctx &c, const double *u, const double *r) {
-  using C = Gj2Cfg<4 * Q * Q, 16 * Q + 1, WR, WC>;
-  auto kern = condense_gj2_kernel<Q, MINB, WR, WC>;
-  EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::DYN));
-  const int grid = std::min(c.n, sm_count_hdg() * MINB);
-  kern<<<grid, C::THREADS, C::DYN, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, r,
-                                                c.XY, c.Cb, c.sf, c.contrib, c.panels, c.derr);
-}
-
 template <int Q>
 static void launch_condense_gjg(Ctx &c, const double *u, const double *r) {
   using C = GjgCfg<Q>;
@@ -1123,43 +941,71 @@ static void launch_condense_gjg(Ctx &c, const double *u, const double *r) {
                                           c.Cb, c.sf, c.contrib, c.panels, c.work_gj, c.derr);
 }
 
-void launch_condense(Ctx &c, const double *u, const double *r) {
-  c.ensure_hdg();
-  const int grid = condense_grid(c);
+template <int Q, int WR, int WC, int MINB>
+static void launch_condense_inv(Ctx &c, const double *u, const double *r) {
+  using C = InvCfg<Q, WR, WC>;
+  constexpr size_t dyn = sizeof(double) * (size_t)(C::REGION + condense_inv_aux<Q, WR, WC>());
+  auto kern = condense_inv_kernel<Q, WR, WC, MINB>;
+  EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+  const int grid = std::min(c.n, sm_count_hdg() * MINB);
+  kern<<<grid, C::THREADS, dyn, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, r, c.XY, c.Cb,
+                                            c.sf, c.contrib, c.panels, c.redo, c.derr + 3);
+}
+
+// rhs_f = contrib_L + contrib_R (s.rhs = 0; rhs[ids] += C y)
+static void launch_condensed_rhs(Ctx &c) {
+  face_combine_kernel<<<(c.nl + 255) / 256, 256, 0, c.stream>>>(c.desc.nx, c.desc.ny, c.t, c.nl, nullptr, c.rhs,
+                                                                c.contrib, -1.0, c.rhs, nullptr);
+  EG_CUDA(cudaGetLastError());
+}
+
+// The cells whose inverse the kernels above could not vouch for, by LU with
+// partial pivoting; `count` of them in c.redo.
+static void condense_redo(Ctx &c, const double *u, const double *r, int count) {
   ProfScope ps(c, EG_K_CONDENSE, 2);
-  switch (c.q) {
-    case 1: launch_condense_gj<1, 1, 1, 8>(c, u, r); break;
-    case 2: launch_condense_gj<2, 1, 2, 6>(c, u, r); break;
-    case 3: launch_condense_gj<3, 2, 2, 4>(c, u, r); break;
-    case 4: launch_condense_gj2<4, 3>(c, u, r); break;
-    case 5: launch_condense_gj2<5, 2>(c, u, r); break;
-    case 6: launch_condense_gj2<6, 1, 4, 4>(c, u, r); break;
-    case 7: launch_condense_gjg<7>(c, u, r); break;
-    case 8: launch_condense_gjg<8>(c, u, r); break;
-    case 9: launch_condense_gjg<9>(c, u, r); break;
-    default:
-      EG_DISPATCH_Q(c.q, {
-        constexpr size_t dyn = condense_dyn_bytes<Q>();
-        auto kern = condense_kernel<Q>;
-        if (dyn > 48 * 1024)
-          EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-        if (condense_mode<Q>() == 2 && (c.work_cell == nullptr || c.work_slots < grid)) {
-          constexpr int M = 4 * Q * Q;
-          c.work_cell = c.alloc_n<double>((size_t)grid * M * M);
-          c.work_slots = grid;
-        }
-        kern<<<grid, 256, dyn, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u,
-                                           r, c.XY, c.Cb, c.sf, c.contrib, c.panels, c.work_cell,
-                                           c.derr);
-      });
+  const int grid = std::min(count, sm_count_hdg());
+  EG_DISPATCH_Q(c.q, {
+    constexpr size_t dyn = condense_dyn_bytes<Q>();
+    auto kern = condense_kernel<Q>;
+    if (dyn > 48 * 1024) EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    if (condense_mode<Q>() == 2 && (c.work_cell == nullptr || c.work_slots < grid)) {
+      constexpr int M = 4 * Q * Q;
+      c.work_cell = c.alloc_n<double>((size_t)grid * M * M);
+      c.work_slots = grid;
+    }
+    kern<<<grid, 256, dyn, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, r, c.XY, c.Cb,
+                                       c.sf, c.contrib, c.panels, c.work_cell, c.redo, count, c.derr);
+  });
+  EG_CUDA(cudaGetLastError());
+  EG_CUDA(cudaMemsetAsync(c.derr + 3, 0, sizeof(int), c.stream));
+  launch_condensed_rhs(c);
+}
+
+void condense(Ctx &c, const double *u, const double *r) {
+  c.ensure_hdg();
+  {
+    ProfScope ps(c, EG_K_CONDENSE, 2);
+    switch (c.q) {
+      case 1: launch_condense_inv<1, 1, 1, 16>(c, u, r); break;
+      case 2: launch_condense_inv<2, 1, 1, 16>(c, u, r); break;
+      case 3: launch_condense_inv<3, 1, 1, 10>(c, u, r); break;
+      case 4: launch_condense_inv<4, 2, 2, 4>(c, u, r); break;
+      case 5: launch_condense_inv<5, 2, 2, 2>(c, u, r); break;
+      case 6: launch_condense_inv<6, 3, 4, 1>(c, u, r); break;
+      case 7: launch_condense_gjg<7>(c, u, r); break;
+      case 8: launch_condense_gjg<8>(c, u, r); break;
+      case 9: launch_condense_gjg<9>(c, u, r); break;
+      default: fail(EG_ERR_INVALID, "unsupported degree");
+    }
+    EG_CUDA(cudaGetLastError());
+    launch_condensed_rhs(c);
   }
-  EG_CUDA(cudaGetLastError());
-  // rhs_f = contrib_L + contrib_R (s.rhs = 0; rhs[ids] += C y)
-  const int blocks = (c.nl + 255) / 256;
-  face_combine_kernel<<<blocks, 256, 0, c.stream>>>(c.desc.nx, c.desc.ny, c.t, c.nl, nullptr, c.rhs,
-                                                    c.contrib, -1.0, c.rhs, nullptr);
-  EG_CUDA(cudaGetLastError());
   c.condensed = true;
+  c.check_device_error();
+  if (const int count = c.herr[3]) {
+    condense_redo(c, u, r, count);
+    c.check_device_error();
+  }
 }
 
 void launch_schur_apply(Ctx &c, const double *v, double *y) {

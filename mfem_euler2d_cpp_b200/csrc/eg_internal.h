@@ -191,6 +191,7 @@ struct Ctx {
   double *rhs = nullptr, *lam = nullptr, *tmp_trace = nullptr;  // nl
   double *work_cell = nullptr;  // global LU workspace for large cells
   int work_slots = 0;
+  int *redo = nullptr;          // n cells a condensation or DG factor solves again by pivoted LU (count in derr[3])
   double *work_gj = nullptr;    // k >= 5 condensation: one m x (m + 4t + 1) slab per CTA
   int work_gj_slots = 0;
   // preconditioners (factored in place): DG n blocks m x m, HDG nf blocks t x t;
@@ -299,7 +300,9 @@ void launch_dg_inverse_apply(Ctx &c, const double *b, double *x);
 // the explicit inverses a record applies, column-major (n m^2 doubles, host)
 void download_dg_record_inverse(Ctx &c, double *dst);
 // ---- launchers (eg_hdg.cu) ----
-void launch_condense(Ctx &c, const double *u, const double *r);
+// condensation of every cell at state u with residual r; synchronises and
+// raises a singular cell
+void condense(Ctx &c, const double *u, const double *r);
 void launch_schur_apply(Ctx &c, const double *v, double *y);
 void launch_recover(Ctx &c, const double *lam, double *du);
 void launch_recovered_residual(Ctx &c, const double *eq, double *er);
