@@ -155,7 +155,7 @@ void Ctx::ensure_krylov() {
 void Ctx::ensure_pc_dg() {
   if (pc_dg) return;
   pc_dg = alloc_n<double>((size_t)n * m * m);
-  piv_dg = alloc_n<int>((size_t)n * m);
+  if (!redo) redo = alloc_n<int>(n);
 }
 void Ctx::ensure_pc_hdg() {
   if (pc_hdg) return;
@@ -186,7 +186,7 @@ struct DgOps : LinearOps {
     if (c.opts.precond == EG_PC_BLOCK_ILU0)
       launch_ilu_apply(c, EG_FORM_DG, b, x);
     else
-      launch_dg_jacobi_apply(c, b, x);
+      launch_dg_inverse_apply(c, b, x);
   }
 };
 struct HdgOps : LinearOps {
@@ -224,7 +224,10 @@ static void pc_factor(Ctx &c, int form, bool factor) {
     // FillBlocks + FixedBlockILU::Factor (src/linear.cpp:191, 196-197)
     ilu_refresh(c, form, factor);
   } else if (form == EG_FORM_DG) {
-    launch_dg_jacobi(c, c.u, factor);
+    if (factor)
+      launch_dg_inverse(c, c.u);
+    else
+      launch_dg_jacobi(c, c.u);
   } else {
     if (!c.condensed) fail(EG_ERR_INVALID, "Schur preconditioner requires a condensation");
     launch_schur_jacobi(c, factor);
@@ -731,13 +734,7 @@ int eg_download(eg_ctx *ctx, int slot, double *dst) {
     if (slot == EG_SLOT_PC_BLOCKS) {
       if (c.opts.form == EG_FORM_DG) {
         if (!c.pc_dg) eg::fail(EG_ERR_INVALID, "no preconditioner built");
-        if (eg::dg_pc_is_record(c)) {
-          // the slot holds the inverses the record applies, column-major
-          if (!dst) eg::fail(EG_ERR_INVALID, "null vector");
-          eg::download_dg_record_inverse(c, dst);
-        } else {
-          eg::download_vec(c, dst, c.pc_dg, (size_t)c.n * c.m * c.m);
-        }
+        eg::download_vec(c, dst, c.pc_dg, (size_t)c.n * c.m * c.m);
       } else {
         if (!c.pc_hdg) eg::fail(EG_ERR_INVALID, "no preconditioner built");
         eg::download_vec(c, dst, c.pc_hdg, (size_t)c.nf * c.t * c.t);
@@ -901,7 +898,7 @@ int eg_pc_apply(eg_ctx *ctx, const double *b, double *x) {
       if (ilu)
         eg::launch_ilu_apply(c, EG_FORM_DG, c.tmp_body, c.er);
       else
-        eg::launch_dg_jacobi_apply(c, c.tmp_body, c.er);
+        eg::launch_dg_inverse_apply(c, c.tmp_body, c.er);
       c.check_device_error();
       eg::download_vec(c, x, c.er, c.nu);
     } else {

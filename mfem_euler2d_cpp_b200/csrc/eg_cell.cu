@@ -506,31 +506,15 @@ __global__ void __launch_bounds__(CellCfg<Q>::THREADS)
   }
 }
 
-template <int Q>
-__host__ __device__ constexpr int lu_rmax() {
-  return (4 * Q * Q + 31) / 32;
-}
-// Cells whose m x m block (plus staging) fits in shared memory.
-template <int Q>
-__host__ __device__ constexpr bool dg_block_in_smem() {
-  return 4 * Q * Q <= 144;
-}
-
 // ------------------------------------------------------ DG block Jacobi
-// Per cell: diagonal block (volume + own-face HLL terms) built at the Newton
-// state, then factored in place with partial pivoting (linear.cpp:198-202).
+// Per cell: diagonal block (volume + own-face HLL terms) at the Newton state
+// (PartialDGOperator::DiagonalBlocks); eg_dginv.cu inverts it.
 template <int Q>
 __global__ void __launch_bounds__(256)
-    dg_jacobi_kernel(Geo g, const double *__restrict__ tab, Frozen fz, const double *__restrict__ u,
-                     double *blocks, int *pivots, bool factor, int *err) {
+    dg_jacobi_kernel(Geo g, const double *__restrict__ tab, Frozen fz, const double *__restrict__ u, double *blocks) {
   constexpr int P = Q * Q, M = 4 * P;
-  constexpr bool SM = dg_block_in_smem<Q>();
   __shared__ STab<Q> st;
   __shared__ double us[M], UT[16 * Q], FM[4 * Q * 16];
-  __shared__ int piv_s[M];
-  __shared__ double inv_piv[M];
-  __shared__ double bcast[2];
-  extern __shared__ double dyn[];
   load_tables<Q>(st, tab);
   for (int e = blockIdx.x; e < g.n; e += gridDim.x) {
     __syncthreads();
@@ -540,149 +524,8 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
     dg_face_matrices<Q>(UT, FM, g, fz, e);
     __syncthreads();
-    double *A = SM ? dyn : blocks + (size_t)e * M * M;
-    build_cell_matrix<Q>(A, M, st, us, FM, g);
-    __syncthreads();
-    if (factor) {
-      const bool ok = cta_lu_solve<lu_rmax<Q>()>(A, M, nullptr, 1, M, 0, piv_s, inv_piv, bcast);
-      if (!ok && threadIdx.x == 0) raise_err(err, DERR_SINGULAR_JACOBI);
-    } else {
-      for (int i = threadIdx.x; i < M; i += blockDim.x) piv_s[i] = i;
-    }
-    __syncthreads();
-    if (SM) {
-      double *dst = blocks + (size_t)e * M * M;
-      for (int i = threadIdx.x; i < M * M; i += blockDim.x) dst[i] = A[i];
-    }
-    for (int i = threadIdx.x; i < M; i += blockDim.x) pivots[(size_t)e * M + i] = piv_s[i];
+    build_cell_matrix<Q>(blocks + (size_t)e * M * M, M, st, us, FM, g);
   }
-}
-
-// --------------------------------------------------------- block LU apply
-// x_b = LU_b^{-1} b_b for every block (one warp per block); Jacobi apply of
-// LinearSolver::Impl::Precondition (src/linear.cpp:66-75).
-__global__ void __launch_bounds__(256) block_apply_kernel(const double *__restrict__ blocks,
-                                                          const int *__restrict__ piv, int nblocks,
-                                                          int bs, const double *__restrict__ b,
-                                                          double *__restrict__ x) {
-  extern __shared__ double xs[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int blk = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (blk >= nblocks) return;
-  double *v = xs + warp * bs;
-  for (int i = lane; i < bs; i += 32) v[i] = b[(size_t)blk * bs + i];
-  __syncwarp();
-  warp_lu_apply(blocks + (size_t)blk * bs * bs, piv + (size_t)blk * bs, bs, v);
-  for (int i = lane; i < bs; i += 32) x[(size_t)blk * bs + i] = v[i];
-}
-
-// The same apply with the block's part of x in registers (lane holds rows
-// lane + 32 r, r < R): sweep steps communicate through shuffles only. Every
-// step reads one column of the factor; those reads do not depend on x, so
-// they are issued PD steps ahead into a register ring (fully unrolled sweeps,
-// static ring slots) and a step no longer waits out a memory latency. Column
-// and row indices are clamped into the block for the loads; only the
-// updates are predicated. The diagonal is applied as a product with its
-// reciprocal.
-template <int R>
-__global__ void __launch_bounds__(256) block_apply_reg_kernel(const double *__restrict__ blocks,
-                                                              const int *__restrict__ piv, int nblocks,
-                                                              int m, const double *__restrict__ b,
-                                                              double *__restrict__ x) {
-  constexpr int S = 32 * R;                             // sweep steps (j >= m are no-ops)
-  constexpr int PD = R == 1 ? 16 : (R == 2 ? 8 : (R <= 4 ? 4 : (R <= 8 ? 2 : 1)));  // columns per chunk
-  extern __shared__ double xs[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int blk = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (blk >= nblocks) return;
-  double *v = xs + (size_t)warp * m;
-  const double *lu = blocks + (size_t)blk * m * m;
-  const int *pv = piv + (size_t)blk * m;
-  for (int i = lane; i < m; i += 32) v[i] = b[(size_t)blk * m + i];
-  __syncwarp();
-  if (lane == 0)
-    for (int i = 0; i < m; ++i) {  // row exchanges of the factorisation, in order
-      const int p = pv[i];
-      if (p != i) {
-        const double t = v[i];
-        v[i] = v[p];
-        v[p] = t;
-      }
-    }
-  __syncwarp();
-  double xr[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) xr[r] = lane + 32 * r < m ? v[lane + 32 * r] : 0.;
-  int rows[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) rows[r] = min(lane + 32 * r, m - 1);
-  auto load_col = [&](double (&dst)[R], int j) {
-    const double *col = lu + (size_t)min(max(j, 0), m - 1) * m;
-#pragma unroll
-    for (int r = 0; r < R; ++r) dst[r] = col[rows[r]];
-  };
-  // columns are read in chunks of PD: the next chunk's loads are issued
-  // before the current chunk's steps (double buffer in registers)
-  double cur[PD][R], nxt[PD][R];
-  // forward: unit lower triangle, columns 0, 1, ...
-#pragma unroll
-  for (int d = 0; d < PD; ++d) load_col(cur[d], d);
-#pragma unroll
-  for (int jb = 0; jb < R; ++jb) {
-#pragma unroll 1
-    for (int cc = 0; cc < 32 / PD; ++cc) {
-      const int j0 = 32 * jb + PD * cc;
-#pragma unroll
-      for (int d = 0; d < PD; ++d) load_col(nxt[d], j0 + PD + d);
-#pragma unroll
-      for (int d = 0; d < PD; ++d) {
-        const int j = j0 + d;
-        const double xj = __shfl_sync(0xffffffffu, xr[jb], PD * cc + d);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int i = lane + 32 * r;
-          xr[r] = (j < m && i > j && i < m) ? xr[r] - cur[d][r] * xj : xr[r];
-        }
-      }
-#pragma unroll
-      for (int d = 0; d < PD; ++d)
-#pragma unroll
-        for (int r = 0; r < R; ++r) cur[d][r] = nxt[d][r];
-    }
-  }
-  // backward: upper triangle with its diagonal, columns S-1, S-2, ...
-#pragma unroll
-  for (int d = 0; d < PD; ++d) load_col(cur[d], S - 1 - d);
-#pragma unroll
-  for (int jb = R - 1; jb >= 0; --jb) {
-#pragma unroll 1
-    for (int cc = 32 / PD - 1; cc >= 0; --cc) {
-      const int jtop = 32 * jb + PD * cc + PD - 1;  // first (highest) column of the chunk
-#pragma unroll
-      for (int d = 0; d < PD; ++d) load_col(nxt[d], jtop - PD - d);
-#pragma unroll
-      for (int d = 0; d < PD; ++d) {
-        const int j = jtop - d;
-        const int jl = PD * cc + PD - 1 - d;  // j % 32
-        // u_jj sits in lane j % 32, register j / 32 (= jb) of this column
-        const double ujj = __shfl_sync(0xffffffffu, cur[d][jb], jl);
-        const double xo = __shfl_sync(0xffffffffu, xr[jb], jl) * (1.0 / ujj);
-        if (j < m && lane == jl) xr[jb] = xo;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int i = lane + 32 * r;
-          xr[r] = (j < m && i < j) ? xr[r] - cur[d][r] * xo : xr[r];
-        }
-      }
-#pragma unroll
-      for (int d = 0; d < PD; ++d)
-#pragma unroll
-        for (int r = 0; r < R; ++r) cur[d][r] = nxt[d][r];
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-    if (lane + 32 * r < m) x[(size_t)blk * m + lane + 32 * r] = xr[r];
 }
 
 // ================================================================ launchers
@@ -782,52 +625,11 @@ static int sm_count() {
   return n;
 }
 
-void launch_dg_jacobi(Ctx &c, const double *u, bool factor) {
-  if (factor && dg_inverse_supported(c.q)) {
-    launch_dg_inverse(c, u);
-    c.dg_pc_inverse = true;
-    return;
-  }
-  c.dg_pc_inverse = false;
+void launch_dg_jacobi(Ctx &c, const double *u) {
   c.ensure_pc_dg();
   ProfScope ps(c, EG_K_DG_JACOBI, 1);
-  EG_DISPATCH_Q(c.q, {
-    constexpr int M = 4 * Q * Q;
-    const size_t dyn = dg_block_in_smem<Q>() ? sizeof(double) * M * M : 0;
-    auto kern = dg_jacobi_kernel<Q>;
-    if (dyn > 48 * 1024)
-      EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    const int grid = std::min(c.n, sm_count() * 8);
-    kern<<<grid, 256, dyn, c.stream>>>(c.geo, c.tab, frozen_of(c), u, c.pc_dg, c.piv_dg, factor, c.derr);
-  });
-  EG_CUDA(cudaGetLastError());
-}
-
-void launch_dg_jacobi_apply(Ctx &c, const double *b, double *x) {
-  if (c.dg_pc_inverse)
-    launch_dg_inverse_apply(c, b, x);
-  else
-    launch_block_apply(c, c.pc_dg, c.piv_dg, c.n, c.m, b, x);
-}
-
-void launch_block_apply(Ctx &c, const double *blocks, const int *piv, int nblocks, int bs,
-                        const double *b, double *x) {
-  // 4 warps (blocks) per CTA: the register-resident sweeps use ~100
-  // registers, so smaller CTAs pack more warps per SM
-  const int warps = 4;
-  const int grid = (nblocks + warps - 1) / warps;
-  const size_t dyn = sizeof(double) * bs * warps;
-  ProfScope ps(c, EG_K_PC_APPLY, 1);
-  switch ((bs + 31) / 32) {
-#define EG_BAR(RR)                                                                                    \
-  case RR:                                                                                            \
-    block_apply_reg_kernel<RR><<<grid, warps * 32, dyn, c.stream>>>(blocks, piv, nblocks, bs, b, x);   \
-    break;
-    EG_BAR(1) EG_BAR(2) EG_BAR(4) EG_BAR(5) EG_BAR(7) EG_BAR(8) EG_BAR(11)
-#undef EG_BAR
-    default:
-      block_apply_kernel<<<grid, warps * 32, dyn, c.stream>>>(blocks, piv, nblocks, bs, b, x);
-  }
+  const int grid = std::min(c.n, sm_count() * 8);
+  EG_DISPATCH_Q(c.q, dg_jacobi_kernel<Q><<<grid, 256, 0, c.stream>>>(c.geo, c.tab, frozen_of(c), u, c.pc_dg));
   EG_CUDA(cudaGetLastError());
 }
 

@@ -36,6 +36,22 @@ __device__ __forceinline__ void dmma_m8n8k4(double &d0, double &d1, double a, do
                : "d"(a), "d"(b));
 }
 
+// Reciprocal of a pivot: hardware estimate refined by two Newton-Raphson
+// steps r <- r + r (1 - x r) (quadratic convergence from the ~2^-20 estimate;
+// result within one unit in the last place of 1/x). The estimate flushes
+// subnormal inputs and results to zero, so magnitudes outside
+// [2^-1020, 2^1020] (and zero, infinities, NaN) take IEEE division instead.
+__device__ __forceinline__ double pivot_reciprocal(double x) {
+  const double ax = fabs(x);
+  if (!(ax >= 0x1p-1020 && ax <= 0x1p+1020)) return 1.0 / x;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  double e = fma(-x, r, 1.0);
+  r = fma(r, e, r);
+  e = fma(-x, r, 1.0);
+  return fma(r, e, r);
+}
+
 // A shared-memory pair that the compiler may not keep in registers for the next
 // column of tiles: those registers hold the matrix.
 __device__ __forceinline__ double2 lds_pair(const double *p) {
@@ -116,7 +132,7 @@ struct Invert8 {
     step<5>();
     step<6>();
     step<7>();
-    const double id = 1. / d;
+    const double id = pivot_reciprocal(d);
     Ti[row * 8 + c0] = v0 * id;
     Ti[row * 8 + c1] = v1 * id;
     __syncwarp();

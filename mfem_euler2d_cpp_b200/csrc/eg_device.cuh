@@ -299,35 +299,4 @@ __device__ bool cta_lu_solve(double *A, int lda, double *B, int ldb, int m, int 
   return true;
 }
 
-// ----------------------------------------------------- warp LU solve (apply)
-// x <- A^{-1} x for a factored m x m block (packed L\U + pivots) held in
-// global memory; x lives in a per-warp shared buffer. Mirrors
-// LUFactors::Solve (interchanges, unit-lower forward, upper backward).
-__device__ __forceinline__ void warp_lu_apply(const double *__restrict__ lu, const int *__restrict__ piv,
-                                              int m, double *x) {
-  const int lane = threadIdx.x & 31;
-  if (lane == 0)
-    for (int i = 0; i < m; ++i) {
-      const int p = piv[i];
-      if (p != i) {
-        const double t = x[i];
-        x[i] = x[p];
-        x[p] = t;
-      }
-    }
-  __syncwarp();
-  for (int j = 0; j < m; ++j) {
-    const double xj = x[j];
-    for (int i = j + 1 + lane; i < m; i += 32) x[i] -= lu[i + (size_t)j * m] * xj;
-    __syncwarp();
-  }
-  for (int j = m - 1; j >= 0; --j) {
-    const double xj = x[j] / lu[j + (size_t)j * m];
-    __syncwarp();
-    if (lane == 0) x[j] = xj;
-    for (int i = lane; i < j; i += 32) x[i] -= lu[i + (size_t)j * m] * xj;
-    __syncwarp();
-  }
-}
-
 }  // namespace eg

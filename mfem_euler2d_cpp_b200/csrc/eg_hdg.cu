@@ -10,9 +10,8 @@
 //              deterministic).
 #include <algorithm>
 
-#include "eg_cellinv.cuh"
 #include "eg_cellmat.cuh"
-#include "eg_gj.cuh"
+#include "eg_condense.cuh"
 #include "eg_internal.h"
 
 namespace eg {
@@ -200,253 +199,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// ------------------------------------------- condensation for k >= 6 (DMMA)
-// The cell system [A | B | r_e] (m x (m + 4t + 1)) does not fit on chip for
-// k >= 6, so it lives in a per-CTA slab of global memory (L2-resident) and is
-// reduced by blocked Gauss-Jordan with virtual partial pivoting in panels of
-// GjgCfg::NB columns:
-//  1. the panel's columns are staged in shared memory and its pivots chosen
-//     column by column exactly as row partial pivoting on the eliminated
-//     column would (largest magnitude among rows not yet used, first index on
-//     ties: the pivots of LUFactors::Factor, src/condensation.cpp:136-140);
-//  2. T = the panel's pivot rows and top = T^-1 W[pivot rows, trailing];
-//  3. one rank-NB update W[r, trailing] -= a_r top on the FP64 tensor cores
-//     (mma.sync m8n8k4), with a_r the row's panel entries, and T_r - e_r for
-//     the panel's own pivot rows, which turns them into the rows of top.
-// After the last panel the right-hand-side columns hold X = A^-1 B and
-// y = A^-1 r_e in pivot order and are written to XY in unknown order.
-template <int Q>
-struct GjgCfg {
-  static constexpr int P = Q * Q, M = 4 * P, T = 4 * Q, NR = 4 * T + 1, NC = M + NR;
-  static constexpr int NB = 16;                      // panel width
-  static constexpr int NPAN = (M + NB - 1) / NB;
-  static constexpr int MT = (M + 7) / 8;            // 8-row tiles
-  static constexpr int RU = 6;                       // row tiles per load round of the update
-  static constexpr size_t SMEM = sizeof(double) * ((size_t)2 * NB * M + (size_t)NB * NC + 2 * NB * NB) +
-                                 sizeof(int) * (size_t)(3 * M + NB);
-  // two CTAs per SM where their shared memory fits (k = 6): one CTA's
-  // serial pivot chain then overlaps the other's trailing update
-  static constexpr int MINB =
-      2 * (SMEM + sizeof(CondenseShared<Q>) + 2048) <= 227 * 1024 ? 2 : 1;
-};
-
-template <int Q>
-__global__ void __launch_bounds__(256, GjgCfg<Q>::MINB)
-    condense_gjg_kernel(Geo g, const double *__restrict__ tab, Frozen fz, const double *__restrict__ u,
-                        const double *__restrict__ r, double *XY, double *Cb, double *sf, double *contrib,
-                        double *panels, double *work, int *err) {
-  using C = GjgCfg<Q>;
-  constexpr int M = C::M, NR = C::NR, NC = C::NC, NB = C::NB;
-  __shared__ CondenseShared<Q> sh;
-  __shared__ int sing;
-  __shared__ double pivval;
-  extern __shared__ __align__(16) double dyn[];
-  double *P0 = dyn;                          // original panel columns  [NB][M]
-  double *Pw = P0 + (size_t)NB * M;          // working panel columns   [NB][M]
-  double *top = Pw + (size_t)NB * M;         // [NB][NC] (trailing width)
-  double *Tm = top + (size_t)NB * NC;        // [NB][2NB] augmented [T | I], row-major
-  int *used = reinterpret_cast<int *>(Tm + 2 * NB * NB);
-  int *pidx = used + M;                      // panel index of a pivot row of this panel, else -1
-  int *piv = pidx + M;                       // pivot row of every column
-  int *prow = piv + M;                       // pivot rows of this panel
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int gq = lane >> 2, tq = lane & 3;
-  double *W = work + (size_t)blockIdx.x * M * NC;  // column-major, ld M
-  load_tables<Q>(sh.st, tab);
-  for (int e = blockIdx.x; e < g.n; e += gridDim.x) {
-    __syncthreads();
-    condense_build<Q>(sh, g, fz, u, r, Cb, sf, W, W + (size_t)M * M, e, M);
-    for (int i = threadIdx.x; i < M; i += blockDim.x) {
-      used[i] = 0;
-      pidx[i] = -1;
-    }
-    if (threadIdx.x == 0) sing = 0;
-    __syncthreads();
-    for (int pan = 0; pan < C::NPAN; ++pan) {
-      const int c0 = pan * NB, nb = min(NB, M - c0), cs = c0 + nb, ntr = NC - cs;
-      // 1. stage the panel; choose its pivots on a working copy
-      for (int o = threadIdx.x; o < NB * M; o += blockDim.x) {
-        const int j = o / M, rr = o % M;
-        const double v = j < nb ? W[(size_t)(c0 + j) * M + rr] : 0.;
-        P0[o] = v;
-        Pw[o] = v;
-      }
-      __syncthreads();
-      for (int j = 0; j < nb; ++j) {
-        if (warp == 0) {
-          // largest |Pw[j][r]| among unused rows, first row on ties, NaN never
-          // chosen: magnitudes compared as IEEE bit patterns (integer compares,
-          // three warp reductions)
-          constexpr unsigned long long kAbs = 0x7fffffffffffffffull, kInf = 0x7ff0000000000000ull;
-          unsigned long long best = 0ull;
-          int bi = M;
-          for (int rr = lane; rr < M; rr += 32) {
-            if (used[rr]) continue;
-            const unsigned long long bits =
-                (unsigned long long)__double_as_longlong(Pw[(size_t)j * M + rr]) & kAbs;
-            if (bits <= kInf && (bi == M || bits > best)) {
-              best = bits;
-              bi = rr;
-            }
-          }
-          const unsigned hi = (unsigned)(best >> 32), lo = (unsigned)best;
-          const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-          const bool c1 = bi < M && hi == mhi;
-          const unsigned mlo = __reduce_max_sync(0xffffffffu, c1 ? lo : 0u);
-          bi = (int)__reduce_min_sync(0xffffffffu, c1 && lo == mlo ? (unsigned)bi : (unsigned)M);
-          if (lane == 0) {
-            const double pv = bi < M ? Pw[(size_t)j * M + bi] : 0.;  // an all-NaN column is singular
-            if (!(fabs(pv) > 0.)) {
-              sing = 1;
-              bi = 0;
-            }
-            pivval = pivot_reciprocal(pv);
-            prow[j] = bi;
-            piv[c0 + j] = bi;
-            used[bi] = 1;
-            pidx[bi] = j;
-          }
-        }
-        __syncthreads();
-        if (sing) break;
-        const int pr = prow[j];
-        const double inv = pivval;  // 1 / pivot
-        const int rest = nb - j - 1;
-        for (int o = threadIdx.x; o < rest * M; o += blockDim.x) {
-          const int jj = j + 1 + o / M, rr = o % M;
-          if (rr != pr) Pw[(size_t)jj * M + rr] -= Pw[(size_t)j * M + rr] * inv * Pw[(size_t)jj * M + pr];
-        }
-        __syncthreads();
-      }
-      if (sing) break;
-      // 2. T^-1 by Gauss-Jordan with partial pivoting on [T | I] (nb x 2nb)
-      for (int o = threadIdx.x; o < NB * 2 * NB; o += blockDim.x) {
-        const int i = o / (2 * NB), k = o % (2 * NB);
-        double v = 0.;
-        if (i < nb && k < nb) v = P0[(size_t)k * M + prow[i]];
-        else if (k >= NB && k - NB == i) v = 1.;
-        else if (i >= nb && k == i) v = 1.;  // identity padding of a partial panel
-        Tm[o] = v;
-      }
-      __syncthreads();
-      if (warp == 0) {
-        for (int j = 0; j < NB; ++j) {
-          // pivot among rows j..NB-1 of column j (lane i holds row i): largest
-          // magnitude, first row on ties, NaN never chosen (row j if all are)
-          constexpr unsigned long long kAbs = 0x7fffffffffffffffull, kInf = 0x7ff0000000000000ull;
-          const unsigned long long bits =
-              lane < NB ? (unsigned long long)__double_as_longlong(Tm[lane * 2 * NB + j]) & kAbs : 0ull;
-          const bool cand = lane >= j && lane < NB && bits <= kInf;
-          const unsigned hi = cand ? (unsigned)(bits >> 32) : 0u, lo = cand ? (unsigned)bits : 0u;
-          const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-          const bool c1 = cand && hi == mhi;
-          const unsigned mlo = __reduce_max_sync(0xffffffffu, c1 ? lo : 0u);
-          const unsigned first = __reduce_min_sync(0xffffffffu, c1 && lo == mlo ? (unsigned)lane : 32u);
-          const int bi = first < 32u ? (int)first : j;
-          const double pv = Tm[bi * 2 * NB + j];
-          __syncwarp();
-          if (bi != j) {  // swap rows j and bi (lane = column)
-            const double a0 = Tm[j * 2 * NB + lane], b0 = Tm[bi * 2 * NB + lane];
-            __syncwarp();
-            Tm[j * 2 * NB + lane] = b0;
-            Tm[bi * 2 * NB + lane] = a0;
-          }
-          __syncwarp();
-          const double ip = 1.0 / pv;
-          Tm[j * 2 * NB + lane] *= ip;
-          __syncwarp();
-          double f[NB];
-#pragma unroll
-          for (int i = 0; i < NB; ++i) f[i] = Tm[i * 2 * NB + j];
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < NB; ++i)
-            if (i != j) Tm[i * 2 * NB + lane] -= f[i] * Tm[j * 2 * NB + lane];
-          __syncwarp();
-        }
-      }
-      // top = T^-1 W[prow, trailing]: gather the pivot rows, then transform in place
-      for (int o = threadIdx.x; o < NB * ntr; o += blockDim.x) {
-        const int k = o / ntr, c = o % ntr;
-        top[(size_t)k * NC + c] = k < nb ? W[(size_t)(cs + c) * M + prow[k]] : 0.;
-      }
-      __syncthreads();
-      for (int c = threadIdx.x; c < ntr; c += blockDim.x) {
-        double wv[NB], out[NB];
-#pragma unroll
-        for (int k = 0; k < NB; ++k) wv[k] = top[(size_t)k * NC + c];
-#pragma unroll
-        for (int i = 0; i < NB; ++i) {
-          double s = 0.;
-#pragma unroll
-          for (int k = 0; k < NB; ++k) s += Tm[i * 2 * NB + NB + k] * wv[k];
-          out[i] = s;
-        }
-#pragma unroll
-        for (int i = 0; i < NB; ++i) top[(size_t)i * NC + c] = i < nb ? out[i] : 0.;
-      }
-      __syncthreads();
-      // 3. rank-NB update of the trailing columns on the tensor cores
-      const int ntile_c = (ntr + 7) / 8;
-      for (int ct = warp; ct < ntile_c; ct += nwarps) {
-        double bf[NB / 4];
-#pragma unroll
-        for (int ks = 0; ks < NB / 4; ++ks) {
-          const int cc = ct * 8 + gq;
-          bf[ks] = cc < ntr ? top[(size_t)(4 * ks + tq) * NC + cc] : 0.;
-        }
-        const int col0 = cs + ct * 8 + 2 * tq;
-        const bool ok0 = col0 < NC, ok1 = col0 + 1 < NC;
-        // GjgCfg::RU row tiles per round: their loads are all in flight before the MMAs
-        for (int rt0 = 0; rt0 < C::MT; rt0 += C::RU) {
-          double cv[C::RU][2];
-#pragma unroll
-          for (int u = 0; u < C::RU; ++u) {
-            const int ra = (rt0 + u) * 8 + gq;  // row of this lane's A fragment and C values
-            const bool rok = ra < M;
-            cv[u][0] = rok && ok0 ? W[(size_t)col0 * M + ra] : 0.;
-            cv[u][1] = rok && ok1 ? W[(size_t)(col0 + 1) * M + ra] : 0.;
-          }
-#pragma unroll
-          for (int u = 0; u < C::RU; ++u) {
-            const int ra = (rt0 + u) * 8 + gq;
-            const bool rok = ra < M;
-            const int pi = rok ? pidx[ra] : -1;
-#pragma unroll
-            for (int ks = 0; ks < NB / 4; ++ks) {
-              const int k = 4 * ks + tq;
-              double a = rok ? P0[(size_t)k * M + ra] : 0.;
-              if (pi == k) a -= 1.;
-              dmma_m8n8k4(cv[u][0], cv[u][1], -a, bf[ks]);
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < C::RU; ++u) {
-            const int ra = (rt0 + u) * 8 + gq;
-            if (ra < M && ok0) W[(size_t)col0 * M + ra] = cv[u][0];
-            if (ra < M && ok1) W[(size_t)(col0 + 1) * M + ra] = cv[u][1];
-          }
-        }
-      }
-      __syncthreads();  // every warp has finished reading pidx for this panel
-      for (int j = threadIdx.x; j < nb; j += blockDim.x) pidx[prow[j]] = -1;
-      __syncthreads();
-    }
-    if (sing) {
-      if (threadIdx.x == 0) raise_err(err, DERR_SINGULAR_CELL);
-      continue;
-    }
-    // right-hand sides back to unknown order: X(j, c) = W(piv[j], M + c)
-    double *R = XY + (size_t)e * M * NR;
-    for (int o = threadIdx.x; o < M * NR; o += blockDim.x) {
-      const int c = o / M, j = o % M;
-      R[o] = W[(size_t)(M + c) * M + piv[j]];
-    }
-    __syncthreads();
-    condense_epilogue<Q>(sh, R, false, XY, contrib, panels, g.npan, e);
-  }
-}
-
 // --------------------------------------- condensation (k <= 5): cell inverses
 // Per cell: A is assembled in shared memory, inverted in registers by the
 // block Gauss-Jordan of eg_cellinv.cuh, and written back; X = A^{-1} B, y and
@@ -455,73 +207,6 @@ __global__ void __launch_bounds__(256, GjgCfg<Q>::MINB)
 // than eliminating the 4t + 1 right-hand sides (2 m^3 against m^3 + 2 m^2
 // (4t + 1): 2.0 against 2.6 M at k = 4), needs no registers for them, and the
 // matrix fits an SM twice at k = 4.
-template <int Q>
-struct CondenseInvShared {
-  static constexpr int M = 4 * Q * Q;
-  STab<Q> st;
-  alignas(16) double us[M], rs[M], y[M], UT[16 * Q], FM[64 * Q], CB[64 * Q], SF[4 * Q], lift[4 * Q * Q];
-  int bad;
-};
-
-// Traces, face matrices FM = sign J(U_own) + stab I (stab = a or b), flux
-// blocks C = -ew FM and lift scalars B = -dt len/|K| ew stab of a cell
-// (src/problem.cpp:622-630, 661-699); the node Jacobians go to J.
-template <int Q>
-__device__ __forceinline__ void condense_cell_data(CondenseInvShared<Q> &sh, const Geo &g, const Frozen &fz,
-                                                   const double *__restrict__ u, const double *__restrict__ r, double *Cb,
-                                                   double *sf_out, double *J, int e) {
-  constexpr int M = 4 * Q * Q;
-  for (int i = threadIdx.x; i < M; i += blockDim.x) {
-    sh.us[i] = u[(size_t)e * M + i];
-    sh.rs[i] = r[(size_t)e * M + i];
-  }
-  if (threadIdx.x == 0) sh.bad = 0;
-  __syncthreads();
-  cell_traces<Q>(sh.st, sh.us, sh.UT);
-  node_jacobians<Q>(J, sh.st, sh.us, g);
-  __syncthreads();
-  for (int task = threadIdx.x; task < 4 * Q; task += blockDim.x) {
-    const int s = task / Q, j = task % Q;
-    const bool L = side_is_left(s);
-    const int fi = cell_face(e, s, g.nx, g.ny) * Q + j;
-    const double stab = L ? fz.a[fi] : fz.b[fi], ewj = sh.st.ew(j), nsign = L ? 1. : -1.;
-    double jm[16];
-    jacobian_axis(sh.UT + 4 * task, s >> 1, g.gm1, jm);
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const double v = nsign * jm[k] + ((k % 5) == 0 ? stab : 0.);
-      sh.FM[task * 16 + k] = v;
-      sh.CB[task * 16 + k] = -ewj * v;
-    }
-    const double sv = -(g.dt * (s < 2 ? g.hy : g.hx) / g.area * ewj) * stab;
-    sh.SF[task] = sv;
-    sf_out[(size_t)e * 4 * Q + task] = sv;
-    for (int l = 0; l < Q; ++l) {
-      const int i = line_node<Q>(s, j, l);
-      sh.lift[task * Q + l] = sh.st.fb(s, j, l) * sh.st.inv_mass(i) * sv;
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 64 * Q; i += blockDim.x) Cb[(size_t)e * 64 * Q + i] = sh.CB[i];
-}
-
-// Row r of V B for the four sides, from a matrix V whose column c starts at V
-// + c * ld: entry jc = 4 jj + c of every side is a weighted sum over the
-// x-line (sides 0, 1) or the y-line (sides 2, 3) through face point jj.
-template <int Q>
-__device__ __forceinline__ void lift_row(const double *lift, const double *V, int ld, int jc, double (&x)[4]) {
-  const int jj = jc >> 2, c = jc & 3;
-  x[0] = x[1] = x[2] = x[3] = 0.;
-#pragma unroll
-  for (int l = 0; l < Q; ++l) {
-    const double vx = V[(size_t)(4 * (jj * Q + l) + c) * ld], vy = V[(size_t)(4 * (l * Q + jj) + c) * ld];
-    x[0] += lift[jj * Q + l] * vx;
-    x[1] += lift[(Q + jj) * Q + l] * vx;
-    x[2] += lift[(2 * Q + jj) * Q + l] * vy;
-    x[3] += lift[(3 * Q + jj) * Q + l] * vy;
-  }
-}
-
 template <int Q, int WR, int WC>
 __host__ __device__ constexpr int condense_inv_aux() {  // doubles of J, later of one side's C R A^{-1}
   constexpr int P = Q * Q, M = 4 * P, T = 4 * Q;
@@ -925,22 +610,6 @@ static int sm_count_hdg() {
   return n;
 }
 
-template <int Q>
-static void launch_condense_gjg(Ctx &c, const double *u, const double *r) {
-  using C = GjgCfg<Q>;
-  auto kern = condense_gjg_kernel<Q>;
-  EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
-  int per_sm = 0;
-  EG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, C::SMEM));
-  const int grid = std::min(c.n, std::max(1, std::min(per_sm, C::MINB)) * sm_count_hdg());
-  if (c.work_gj == nullptr || c.work_gj_slots < grid) {
-    c.work_gj = c.alloc_n<double>((size_t)grid * C::M * C::NC);
-    c.work_gj_slots = grid;
-  }
-  kern<<<grid, 256, C::SMEM, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, r, c.XY,
-                                          c.Cb, c.sf, c.contrib, c.panels, c.work_gj, c.derr);
-}
-
 template <int Q, int WR, int WC, int MINB>
 static void launch_condense_inv(Ctx &c, const double *u, const double *r) {
   using C = InvCfg<Q, WR, WC>;
@@ -992,10 +661,7 @@ void condense(Ctx &c, const double *u, const double *r) {
       case 4: launch_condense_inv<4, 2, 2, 4>(c, u, r); break;
       case 5: launch_condense_inv<5, 2, 2, 2>(c, u, r); break;
       case 6: launch_condense_inv<6, 3, 4, 1>(c, u, r); break;
-      case 7: launch_condense_gjg<7>(c, u, r); break;
-      case 8: launch_condense_gjg<8>(c, u, r); break;
-      case 9: launch_condense_gjg<9>(c, u, r); break;
-      default: fail(EG_ERR_INVALID, "unsupported degree");
+      default: launch_condense_cluster(c, u, r);
     }
     EG_CUDA(cudaGetLastError());
     launch_condensed_rhs(c);

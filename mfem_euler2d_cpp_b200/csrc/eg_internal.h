@@ -192,16 +192,11 @@ struct Ctx {
   double *work_cell = nullptr;  // global LU workspace for large cells
   int work_slots = 0;
   int *redo = nullptr;          // n cells a condensation or DG factor solves again by pivoted LU (count in derr[3])
-  double *work_gj = nullptr;    // k >= 5 condensation: one m x (m + 4t + 1) slab per CTA
+  double *work_gj = nullptr;    // k >= 6 condensation: one m x m inverse per cluster
   int work_gj_slots = 0;
-  // preconditioners (factored in place): DG n blocks m x m, HDG nf blocks t x t;
-  // dg_pc_inverse: pc_dg holds explicit inverses (column-major, k <= 2) or a
-  // Gauss-Jordan record (k = 3..5, with dg_rec_fac and dg_rec_pivs), else
-  // pivoted LU
+  // block Jacobi: explicit inverses (or, unfactored, the blocks), column-major:
+  // DG n blocks m x m, HDG nf blocks t x t
   double *pc_dg = nullptr, *pc_hdg = nullptr;
-  bool dg_pc_inverse = false;
-  double *dg_rec_fac = nullptr;
-  int *dg_rec_pivs = nullptr;
   // DG partial assembly (launch_dg_refresh): dt w J_x, dt w J_y per cell node
   // and lw J(U_L) + pen I, rw J(U_R) - pen I per face point, component-major
   double *dgc_vol = nullptr, *dgc_face = nullptr;
@@ -210,7 +205,7 @@ struct Ctx {
   double *dense_a = nullptr;
   int *dense_piv = nullptr;
   int dense_n = 0;
-  int *piv_dg = nullptr, *piv_hdg = nullptr;
+  int *piv_hdg = nullptr;
   // Krylov workspace (size N = max(nu, nl) so both forms share it)
   int kN = 0, kR = 0;
   double *V = nullptr;
@@ -283,26 +278,19 @@ void launch_dg_apply_cached(Ctx &c, const double *x, double *y);
 constexpr int kDenseMaxUnknowns = 5000;
 void dense_factor(Ctx &c, int form);  // LU of the assembled blocks of c.ilu[form]
 void dense_solve(Ctx &c, const double *b, double *x);
-void launch_dg_jacobi(Ctx &c, const double *u, bool factor);
-void launch_block_apply(Ctx &c, const double *blocks, const int *piv, int nblocks, int bs,
-                        const double *b, double *x);
-// DG block-Jacobi apply x = J_KK^{-1} b with whichever factors the last
-// launch_dg_jacobi(factor = true) formed (explicit inverses or pivoted LU).
-void launch_dg_jacobi_apply(Ctx &c, const double *b, double *x);
-// ---- explicit DG block-Jacobi inverses (eg_dginv.cu) ----
-bool dg_inverse_supported(int q);
-// k <= 2: pc_dg holds the column-major J_KK^{-1}; k = 3..5: the Gauss-Jordan
-// record (pc_dg: reduced block, dg_rec_fac: panel T^{-1}, dg_rec_pivs: panel
-// pivot rows, piv_dg: unknown order of the result rows)
-bool dg_pc_is_record(const Ctx &c);
+void launch_dg_jacobi(Ctx &c, const double *u);  // the unfactored cell blocks to pc_dg
+// ---- explicit DG block-Jacobi inverses, column-major in pc_dg (eg_dginv.cu) ----
+// synchronises and raises a singular block
 void launch_dg_inverse(Ctx &c, const double *u);
 void launch_dg_inverse_apply(Ctx &c, const double *b, double *x);
-// the explicit inverses a record applies, column-major (n m^2 doubles, host)
-void download_dg_record_inverse(Ctx &c, double *dst);
 // ---- launchers (eg_hdg.cu) ----
 // condensation of every cell at state u with residual r; synchronises and
 // raises a singular cell
 void condense(Ctx &c, const double *u, const double *r);
+// k >= 6: one thread-block cluster per cell (eg_cluster.cu); the second writes
+// the explicit DG block-Jacobi inverses to pc_dg
+void launch_condense_cluster(Ctx &c, const double *u, const double *r);
+void launch_dg_inverse_cluster(Ctx &c, const double *u);
 void launch_schur_apply(Ctx &c, const double *v, double *y);
 void launch_recover(Ctx &c, const double *lam, double *du);
 void launch_recovered_residual(Ctx &c, const double *eq, double *er);
