@@ -188,6 +188,13 @@ struct DgOps : LinearOps {
     else
       launch_dg_inverse_apply(c, b, x);
   }
+  bool fused(const Ctx &c, int R) const override {
+    return c.opts.assembly == EG_ASSEMBLY_PARTIAL && fused_solve_supported(c, R);
+  }
+  double solve_fused(Ctx &c, const KrylovBufs<double> &kb, const double *rhs, double *x, double tol, int limit,
+                     bool zero_guess, double rhs_norm, int *count) override {
+    return fused_solve_dg(c, kb, rhs, x, tol, limit, zero_guess, rhs_norm, count);
+  }
 };
 struct HdgOps : LinearOps {
   explicit HdgOps(Ctx &c) {

@@ -9,8 +9,9 @@
 // of the step is that latency.
 //
 // One step, with CTA b owning the cells [e0, e1) and the vector entries of
-// those cells (HDG: their faces 2e and 2e + 1):
-//   operator    contributions of the CTA's cells            | grid barrier
+// those cells (HDG: their faces 2e and 2e + 1; DG: their nodes):
+//   operator    contributions of the CTA's cells (HDG) or
+//               values of its faces (DG), then its cells    | grid barrier
 //   pass 1      w = A z on the CTA's entries; V^T M w        | grid barrier
 //   pass 2      w -= V h; V^T M w and w^T M w                | grid barrier
 //   pass 3      w -= V h2; V_{j+1} = w / |w|; z = P V_{j+1}  | grid barrier
@@ -238,7 +239,7 @@ struct HdgOp {
     return res;
   }
   // contributions of the cells [e0, e1) for the trace vector x
-  static __device__ __forceinline__ bool apply(const Args &a, Shared &sh, const T *x, int e0, int e1,
+  static __device__ __forceinline__ bool apply(const Args &a, Shared &sh, const T *x, T *, int e0, int e1,
                                                const GridBar &bar, unsigned &target) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int S = a.split, slots = kGW / S, slice = warp % S, slot = warp / S;
@@ -341,7 +342,8 @@ struct HdgOp {
            __ldcg(a.contrib + (size_t)R * K + rs * TT + r);
   }
   // z = P v on the entries [i0, i1) (whole blocks); v was written by this CTA
-  static __device__ __forceinline__ void precondition(const Args &a, Shared &, const T *v, T *z, int i0, int i1) {
+  static __device__ __forceinline__ void precondition(const Args &a, Shared &, const T *v, T *z, int, int, int i0,
+                                                      int i1) {
     for (int i = i0 + (int)threadIdx.x; i < i1; i += blockDim.x) {
       const int f = i / TT, r = i % TT;
       const T *inv = a.pc + (size_t)f * TT * TT + r, *b = v + (size_t)f * TT;
@@ -349,6 +351,204 @@ struct HdgOp {
 #pragma unroll
       for (int c = 0; c < TT; ++c) acc += __ldcs(inv + c * TT) * b[c];
       __stcg(z + i, acc);
+    }
+  }
+};
+
+// DG partial assembly (the cached Jacobians of dg_refresh_*_kernel, eg_cell.cu)
+// and explicit cell-block inverses. The face values of the CTA's own faces come
+// first (each face point once), a grid barrier, then the cells, whose values
+// stay in w. S warps share a cell's inverse, as above.
+template <int Q>
+struct DgOp {
+  using Real = double;
+  static constexpr int P = Q * Q, M = 4 * P, CPB = (kGT / P) < 64 ? kGT / P : 64;
+  static constexpr int R2 = (M / 2 + 31) / 32;  // row pairs per lane
+  struct Args {
+    Geo g;
+    const double *tab, *vol, *face, *inv;
+    double *hface;
+    int split;  // S
+  };
+  struct Shared {
+    double fb[4 * P], tdx[P], tdy[P], im[P], ew[Q];
+    union {
+      struct {
+        double fx[CPB][P][4], fy[CPB][P][4], hs[CPB][4 * Q][4];
+      } cell;
+      struct {
+        double v[kGW][M], part[kGW][M];
+      } pc;
+    };
+  };
+  static __device__ __forceinline__ void setup(const Args &a, Shared &sh) {
+    using L = TabLayout<Q>;
+    for (int i = threadIdx.x; i < 4 * P; i += blockDim.x) sh.fb[i] = a.tab[L::FB + i];
+    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+      sh.tdx[i] = a.tab[L::TDX + i];
+      sh.tdy[i] = a.tab[L::TDY + i];
+      sh.im[i] = a.tab[L::IM + i];
+    }
+    for (int i = threadIdx.x; i < Q; i += blockDim.x) sh.ew[i] = a.tab[L::EW + i];
+  }
+  // trace of x on side s of cell c at face point j
+  static __device__ __forceinline__ void trace(const Shared &sh, const double *x, int c, int s, int j, double (&o)[4]) {
+    const double2 *cell = reinterpret_cast<const double2 *>(x + (size_t)c * M);
+    o[0] = o[1] = o[2] = o[3] = 0.;
+#pragma unroll
+    for (int l = 0; l < Q; ++l) {
+      const double f = sh.fb[(s * Q + j) * Q + l];
+      const int node = line_node<Q>(s, j, l);
+      const double2 v0 = __ldcg(cell + 2 * node), v1 = __ldcg(cell + 2 * node + 1);
+      o[0] += f * v0.x;
+      o[1] += f * v0.y;
+      o[2] += f * v1.x;
+      o[3] += f * v1.y;
+    }
+  }
+  static __device__ __forceinline__ bool apply(const Args &a, Shared &sh, const double *x, double *w, int e0, int e1,
+                                               const GridBar &bar, unsigned &target) {
+    const Geo &g = a.g;
+    const long long nq = (long long)g.nf * Q, np = (long long)g.n * P;
+    for (int idx = 2 * e0 * Q + (int)threadIdx.x; idx < 2 * e1 * Q; idx += blockDim.x) {
+      const int f = idx / Q, j = idx % Q, L = f >> 1, axis = f & 1, sl = axis ? 3 : 1;
+      double cf[32];
+#pragma unroll
+      for (int k = 0; k < 32; ++k) cf[k] = __ldcs(a.face + k * nq + idx);
+      double xl[4], xr[4], h[4] = {0., 0., 0., 0.};
+      trace(sh, x, L, sl, j, xl);
+      trace(sh, x, neighbour(L, sl, g.nx, g.ny), sl - 1, j, xr);
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) h[r] += cf[r + 4 * c] * xl[c] + cf[16 + r + 4 * c] * xr[c];
+      const double scale = g.dt * (axis == 0 ? g.hy : g.hx) / g.area * sh.ew[j];
+      double2 *o = reinterpret_cast<double2 *>(a.hface) + (size_t)idx * 2;
+      __stcg(o, make_double2(scale * h[0], scale * h[1]));
+      __stcg(o + 1, make_double2(scale * h[2], scale * h[3]));
+    }
+    if (!grid_barrier(bar, target)) return false;
+    const int lc = threadIdx.x / P, node = threadIdx.x % P, ix = node % Q, iy = node / Q;
+    for (int eb = e0; eb < e1; eb += CPB) {
+      const int e = eb + lc;
+      const bool on = lc < CPB && e < e1;
+      double xx[4];
+      if (on) {
+        const double2 *xv = reinterpret_cast<const double2 *>(x + (size_t)e * M + 4 * node);
+        const double2 x0 = __ldcg(xv), x1 = __ldcg(xv + 1);
+        xx[0] = x0.x;
+        xx[1] = x0.y;
+        xx[2] = x1.x;
+        xx[3] = x1.y;
+        const long long idx = (long long)e * P + node;
+        double fx[4] = {0., 0., 0., 0.}, fy[4] = {0., 0., 0., 0.};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            fx[r] += __ldcs(a.vol + (r + 4 * c) * np + idx) * xx[c];
+            fy[r] += __ldcs(a.vol + (16 + r + 4 * c) * np + idx) * xx[c];
+          }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          sh.cell.fx[lc][node][c] = fx[c];
+          sh.cell.fy[lc][node][c] = fy[c];
+        }
+        for (int task = node; task < 4 * Q; task += P) {
+          const int s = task / Q, j = task % Q;
+          const double2 *h = reinterpret_cast<const double2 *>(a.hface) + ((size_t)cell_face(e, s, g.nx, g.ny) * Q + j) * 2;
+          const double2 h0 = __ldcg(h), h1 = __ldcg(h + 1);
+          const double sg = side_is_left(s) ? 1. : -1.;
+          sh.cell.hs[lc][task][0] = sg * h0.x;
+          sh.cell.hs[lc][task][1] = sg * h0.y;
+          sh.cell.hs[lc][task][2] = sg * h1.x;
+          sh.cell.hs[lc][task][3] = sg * h1.y;
+        }
+      }
+      __syncthreads();
+      if (on) {
+        double acc[4] = {0., 0., 0., 0.};
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+          const double dx = sh.tdx[k * Q + ix], dy = sh.tdy[k * Q + iy];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[c] += dx * sh.cell.fx[lc][iy * Q + k][c] + dy * sh.cell.fy[lc][k * Q + ix][c];
+        }
+        const double w0 = sh.fb[iy * Q + ix], w1 = sh.fb[(Q + iy) * Q + ix], w2 = sh.fb[(2 * Q + ix) * Q + iy],
+                     w3 = sh.fb[(3 * Q + ix) * Q + iy], im = sh.im[node];
+        double o[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const double fc = w0 * sh.cell.hs[lc][iy][c] + w1 * sh.cell.hs[lc][Q + iy][c] +
+                            w2 * sh.cell.hs[lc][2 * Q + ix][c] + w3 * sh.cell.hs[lc][3 * Q + ix][c];
+          o[c] = im * (fc - acc[c]) + xx[c];
+        }
+        double2 *wv = reinterpret_cast<double2 *>(w + (size_t)e * M + 4 * node);
+        wv[0] = make_double2(o[0], o[1]);
+        wv[1] = make_double2(o[2], o[3]);
+      }
+      __syncthreads();
+    }
+    return true;
+  }
+  static __device__ __forceinline__ double value(const Args &, const double *, const double *w, int i) { return w[i]; }
+  static __device__ __forceinline__ void precondition(const Args &a, Shared &sh, const double *v, double *z, int e0,
+                                                      int e1, int, int) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int S = a.split, slots = kGW / S, slice = warp % S, slot = warp / S;
+    const int kper = (M + S - 1) / S, k0 = min(M, slice * kper), k1 = min(M, k0 + kper);
+    const int rounds = (e1 - e0 + slots - 1) / slots;
+    for (int rd = 0; rd < rounds; ++rd) {
+      const int e = e0 + rd * slots + slot;
+      const bool on = e < e1;
+      double acc[R2][2];
+      if (on) {
+        double *sv = sh.pc.v[warp];
+        for (int i = k0 + lane; i < k1; i += 32) sv[i] = v[(size_t)e * M + i];
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < R2; ++r) acc[r][0] = acc[r][1] = 0.;
+        const double2 *A = reinterpret_cast<const double2 *>(a.inv + (size_t)e * M * M);
+#pragma unroll R2 <= 2 ? 8 : 4
+        for (int k = k0; k < k1; ++k) {
+          const double xv = sv[k];
+#pragma unroll
+          for (int r = 0; r < R2; ++r)
+            if (lane + 32 * r < M / 2) {
+              const double2 m = __ldcs(A + (size_t)k * (M / 2) + lane + 32 * r);
+              acc[r][0] = fma(m.x, xv, acc[r][0]);
+              acc[r][1] = fma(m.y, xv, acc[r][1]);
+            }
+        }
+      }
+      if (S == 1) {
+        if (on) {
+#pragma unroll
+          for (int r = 0; r < R2; ++r)
+            if (lane + 32 * r < M / 2)
+              __stcg(reinterpret_cast<double2 *>(z + (size_t)e * M) + lane + 32 * r, make_double2(acc[r][0], acc[r][1]));
+        }
+        __syncwarp();
+        continue;
+      }
+      // the S warps of a cell meet at a barrier of their own
+      if (on) {
+#pragma unroll
+        for (int r = 0; r < R2; ++r)
+          if (lane + 32 * r < M / 2)
+            *reinterpret_cast<double2 *>(&sh.pc.part[warp][2 * (lane + 32 * r)]) = make_double2(acc[r][0], acc[r][1]);
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(32 * S) : "memory");
+      if (on)
+        for (int i = slice * 32 + lane; i < M; i += 32 * S) {
+          double t[2] = {sh.pc.part[slot * S][i], sh.pc.part[slot * S + 1][i]};
+          for (int k = 2; k < S; k += 2) {
+            t[0] += sh.pc.part[slot * S + k][i];
+            t[1] += sh.pc.part[slot * S + k + 1][i];
+          }
+          __stcg(z + (size_t)e * M + i, t[0] + t[1]);
+        }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(32 * S) : "memory");
     }
   }
 };
@@ -462,7 +662,8 @@ template <class Op>
 __global__ void __launch_bounds__(kGT, 1) gmres_kernel(typename Op::Args oa, SolveArgs<typename Op::Real> s) {
   using T = typename Op::Real;
   __shared__ SolveShared sh;
-  __shared__ typename Op::Shared osh;
+  extern __shared__ __align__(16) unsigned char dyn[];
+  typename Op::Shared &osh = *reinterpret_cast<typename Op::Shared *>(dyn);
   const int G = gridDim.x, b = blockIdx.x;
   const int e0 = (int)((long long)s.cells * b / G), e1 = (int)((long long)s.cells * (b + 1) / G);
   const int i0 = e0 * s.per_cell, i1 = e1 * s.per_cell;
@@ -474,7 +675,7 @@ __global__ void __launch_bounds__(kGT, 1) gmres_kernel(typename Op::Args oa, Sol
   __syncthreads();
   // res = rhs - A x for a given guess; norm over the grid
   const auto true_residual = [&](double &norm) -> bool {
-    if (!Op::apply(oa, osh, s.x, e0, e1, s.bar, target)) return false;
+    if (!Op::apply(oa, osh, s.x, s.w, e0, e1, s.bar, target)) return false;
     double nrm = 0.;
     for (int i = i0 + (int)threadIdx.x; i < i1; i += blockDim.x) {
       const T r = s.rhs[i] - Op::value(oa, s.x, s.w, i);
@@ -506,12 +707,12 @@ __global__ void __launch_bounds__(kGT, 1) gmres_kernel(typename Op::Args oa, Sol
     for (int i = threadIdx.x; i <= kGC; i += blockDim.x) sh.g[i] = i == 0 ? beta : 0.;
     for (int i = i0 + (int)threadIdx.x; i < i1; i += blockDim.x) s.V[i] = (T)((double)s.res[i] * inv_beta);
     __syncthreads();
-    Op::precondition(oa, osh, s.V, s.z, i0, i1);
+    Op::precondition(oa, osh, s.V, s.z, e0, e1, i0, i1);
     if (!grid_barrier(s.bar, target)) return;
     int count = 0;
     for (int j = 0; j < s.R && iterations < s.limit; ++j) {
       const int nc = j + 1;
-      if (!Op::apply(oa, osh, s.z, e0, e1, s.bar, target)) return;
+      if (!Op::apply(oa, osh, s.z, s.w, e0, e1, s.bar, target)) return;
       EG_BY_COLUMNS(nc, (cgs_pass<NC, 0, Op>(sh, oa, s.z, s.w, s.V, s.ldv, nc, i0, i1, s.period, part0)));
       if (!grid_barrier(s.bar, target)) return;
       collect_columns(nc, part0, sh.h1);
@@ -557,7 +758,7 @@ __global__ void __launch_bounds__(kGT, 1) gmres_kernel(typename Op::Args oa, Sol
       ++iterations;
       count = nc;
       if (sh.stop || nc == s.R || iterations == s.limit) break;
-      Op::precondition(oa, osh, vnext, s.z, i0, i1);
+      Op::precondition(oa, osh, vnext, s.z, e0, e1, i0, i1);
       if (!grid_barrier(s.bar, target)) return;
     }
     if (err) break;
@@ -580,7 +781,7 @@ __global__ void __launch_bounds__(kGT, 1) gmres_kernel(typename Op::Args oa, Sol
     }
     __syncthreads();
     // z is free here: the last apply of this cycle is behind a barrier
-    Op::precondition(oa, osh, s.comb, s.z, i0, i1);
+    Op::precondition(oa, osh, s.comb, s.z, e0, e1, i0, i1);
     __syncthreads();
     for (int i = i0 + (int)threadIdx.x; i < i1; i += blockDim.x) s.x[i] += __ldcg(s.z + i);
     if (!grid_barrier(s.bar, target)) return;
@@ -631,7 +832,10 @@ double launch_solve(Ctx &c, typename Op::Args &oa, SolveArgs<typename Op::Real> 
   {
     ProfScope ps(c, EG_K_KRYLOV, 1);
     void *params[] = {&oa, &s};
-    EG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(gmres_kernel<Op>), grid, kGT, params, 0,
+    constexpr size_t dyn = sizeof(typename Op::Shared);
+    if (dyn > 32 * 1024)
+      EG_CUDA(cudaFuncSetAttribute(gmres_kernel<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    EG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(gmres_kernel<Op>), grid, kGT, params, dyn,
                                         c.stream));
   }
   EG_CUDA(cudaMemcpyAsync(c.hctl, c.ctl, sizeof(GmresCtl), cudaMemcpyDeviceToHost, c.stream));
@@ -688,6 +892,26 @@ double solve_hdg(Ctx &c, const KrylovBufs<T> &kb, const T *act, const T *D, cons
   return launch_solve<Op>(c, oa, s, grid, count);
 }
 
+template <int Q>
+double solve_dg(Ctx &c, const KrylovBufs<double> &kb, const double *rhs, double *x, double tol, int limit,
+                bool zero_guess, double rhs_norm, int *count) {
+  using Op = DgOp<Q>;
+  if (!c.dgc_h) c.dgc_h = c.alloc_n<double>((size_t)4 * c.nf * c.q);
+  const int grid = solve_grid(c.n, 8. * c.n * ((double)c.m * c.m + 32 * c.p + 64 * c.q), c.nu);
+  const int per = (c.n + grid - 1) / grid;
+  // warps per cell of the block apply: the fewest whose last round of cells
+  // wastes less than a twentieth of the warps
+  int split = 1;
+  while (split < kGW && 20 * (((per * split + kGW - 1) / kGW) * kGW - per * split) > per * split) split *= 2;
+  typename Op::Args oa{c.geo, c.tab, c.dgc_vol, c.dgc_face, c.pc_dg, c.dgc_h, split};
+  SolveArgs<double> s = solve_args(c, kb, rhs, x, tol, limit, zero_guess, rhs_norm, c.nu);
+  s.cells = c.n;
+  s.per_cell = c.m;
+  s.period = c.m;
+  s.mtab = c.mtab_dg;
+  return launch_solve<Op>(c, oa, s, grid, count);
+}
+
 template <class T>
 double solve_hdg_q(Ctx &c, const KrylovBufs<T> &kb, const T *act, const T *D, const T *pc, T *contrib, const T *rhs,
                    T *x, double tol, int limit, bool zero_guess, double rhs_norm, int *count) {
@@ -716,6 +940,11 @@ double fused_solve_hdg(Ctx &c, const KrylovBufs<double> &kb, const double *rhs, 
                        bool zero_guess, double rhs_norm, int *count) {
   return solve_hdg_q<double>(c, kb, c.geo.npan == 16 ? c.panels : c.XY, c.D, c.pc_hdg, c.contrib, rhs, x, tol, limit,
                              zero_guess, rhs_norm, count);
+}
+double fused_solve_dg(Ctx &c, const KrylovBufs<double> &kb, const double *rhs, double *x, double tol, int limit,
+                      bool zero_guess, double rhs_norm, int *count) {
+  EG_DISPATCH_Q(c.q, return solve_dg<Q>(c, kb, rhs, x, tol, limit, zero_guess, rhs_norm, count));
+  fail(EG_ERR_INVALID, "unsupported degree");
 }
 double fused_solve_hdg_f32(Ctx &c, const KrylovBufs<float> &kb, const float *rhs, float *x, double tol, int limit,
                            double rhs_norm, int *count) {

@@ -351,6 +351,9 @@ bool fused_solve_supported(const Ctx &c, int R);
 // leaves rhs - A x in kb.res and returns its weighted norm.
 double fused_solve_hdg(Ctx &c, const KrylovBufs<double> &kb, const double *rhs, double *x, double tol, int limit,
                        bool zero_guess, double rhs_norm, int *count);
+// the same for the DG system with the cached partial assembly and pc_dg
+double fused_solve_dg(Ctx &c, const KrylovBufs<double> &kb, const double *rhs, double *x, double tol, int limit,
+                      bool zero_guess, double rhs_norm, int *count);
 double fused_solve_hdg_f32(Ctx &c, const KrylovBufs<float> &kb, const float *rhs, float *x, double tol, int limit,
                            double rhs_norm, int *count);
 // ---- eg_api.cu ----

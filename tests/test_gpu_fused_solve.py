@@ -5,7 +5,7 @@ inside the solve, a non-zero guess and the bounded waits.
 
 The solve stops when the weighted residual is below 1e-12 of the weighted
 right-hand side. The weights len / ew_j differ by less than 1e2 within a
-mesh used here, so the plain 2-norm ratio, formed with the separate operator
+mesh used here (the DG form: the Gauss weights), so the plain 2-norm ratio, formed with the separate operator
 kernels, is below 1e-10."""
 import numpy as np
 import pytest
@@ -52,6 +52,17 @@ def test_hdg_solution_satisfies_the_separate_operator(nx, ny, k, precision):
         # from a perturbed solution (non-zero guess), without a new factor
         y, _, _ = ctx.linear_solve(rhs, x0=x * (1 + 1e-6), refresh=False)
         assert _rel_residual(ctx, capi.FORM_HDG, y, rhs) < 1e-10
+
+
+@pytest.mark.parametrize("nx,ny,k", [(2, 2, 0), (63, 45, 1), (13, 11, 2), (37, 9, 3), (7, 5, 4), (11, 7, 6), (3, 2, 8)])
+def test_dg_solution_satisfies_the_separate_operator(nx, ny, k):
+    with _context(nx, ny, k, form=capi.FORM_DG) as ctx:
+        rhs = np.cos(0.3 * np.arange(ctx.nu)) + 0.2
+        x, _, st = ctx.linear_solve(rhs)
+        assert st.count > 0 and st.residual <= 1e-12
+        assert _rel_residual(ctx, capi.FORM_DG, x, rhs) < 1e-10
+        y, _, _ = ctx.linear_solve(rhs, x0=x * (1 + 1e-6), refresh=False)
+        assert _rel_residual(ctx, capi.FORM_DG, y, rhs) < 1e-10
 
 
 @pytest.mark.parametrize("restart", [1, 5, 24, 30])
