@@ -111,9 +111,17 @@ void Ctx::prof_resolve() {
   prof.pending.clear();
 }
 
-void Ctx::check_device_error() {
-  EG_CUDA(cudaMemcpyAsync(herr, derr, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream));
+void Ctx::fetch_status() {
+  EG_CUDA(cudaMemcpyAsync(herr, derr, 4 * sizeof(int) + DS_COUNT * sizeof(double), cudaMemcpyDeviceToHost, stream));
   sync();
+}
+
+void Ctx::check_device_error() {
+  fetch_status();
+  raise_device_error();
+}
+
+void Ctx::raise_device_error() {
   if (herr[2]) {
     broken = true;
     fail(EG_ERR_CONTEXT_LOST, kMessages[EG_ERR_CONTEXT_LOST]);
@@ -231,10 +239,11 @@ static void pc_factor(Ctx &c, int form, bool factor) {
     // FillBlocks + FixedBlockILU::Factor (src/linear.cpp:191, 196-197)
     ilu_refresh(c, form, factor);
   } else if (form == EG_FORM_DG) {
-    if (factor)
-      launch_dg_inverse(c, c.u);
-    else
-      launch_dg_jacobi(c, c.u);
+    if (factor) {
+      launch_dg_inverse(c, c.u);  // checks for itself
+      return;
+    }
+    launch_dg_jacobi(c, c.u);
   } else {
     if (!c.condensed) fail(EG_ERR_INVALID, "Schur preconditioner requires a condensation");
     launch_schur_jacobi(c, factor);
@@ -248,8 +257,10 @@ struct LinearOut {
   int count = 0;
   double residual = 0., rhs_norm = 0., assembly = 0., setup = 0., solve = 0.;
 };
+// known_rhs_norm >= 0: the weighted norm of rhs; factored: the preconditioner
+// is up to date although refresh is set.
 static void linear_solve(Ctx &c, int form, const double *rhs, double *x, double *eq, bool refresh,
-                         double tol, LinearOut &out) {
+                         double tol, LinearOut &out, double known_rhs_norm = -1., bool factored = false) {
   DgOps dg(c);
   HdgOps hdg(c);
   LinearOps &ops = form == EG_FORM_DG ? static_cast<LinearOps &>(dg) : static_cast<LinearOps &>(hdg);
@@ -257,7 +268,7 @@ static void linear_solve(Ctx &c, int form, const double *rhs, double *x, double 
   // the residual and work vectors below live in the Krylov workspace, which
   // the dense solve needs as well
   c.ensure_krylov();
-  const double rhs_norm = wnorm(c, rhs, ops.N, ops.mtab, ops.period);
+  const double rhs_norm = known_rhs_norm >= 0. ? known_rhs_norm : wnorm(c, rhs, ops.N, ops.mtab, ops.period);
   out.rhs_norm = rhs_norm;
   if (rhs_norm == 0.) {
     launch_fill(c, ops.N, 0., x);
@@ -281,7 +292,7 @@ static void linear_solve(Ctx &c, int form, const double *rhs, double *x, double 
   if (refresh) {
     if (dense)
       dense_factor(c, form);  // src/linear.cpp:204-206 (no preconditioner)
-    else
+    else if (!factored)
       pc_factor(c, form, true);
   }
   out.setup = now_s() - t0;
@@ -305,7 +316,8 @@ static void linear_solve(Ctx &c, int form, const double *rhs, double *x, double 
     c.check_device_error();  // a preconditioner failure on the device explains the breakdown
     throw;
   }
-  c.check_device_error();
+  // the one-launch solve has checked for itself, and nothing was launched since
+  if (dense || mixed || !ops.fused(c, c.kR)) c.check_device_error();
   out.solve = now_s() - t0;
   out.count = count;
   if (c.opts.assembly == EG_ASSEMBLY_FULL) {
@@ -337,44 +349,79 @@ void newton_update(Ctx &c, double residual_norm, double old_norm, eg_update_stat
   if (!c.update_timer_open) open_update_timer(c);
   const int form = c.opts.form;
   const double eps = std::numeric_limits<double>::epsilon();
-  const double allowance = 128 * eps * (cell_norm(c, c.u) + old_norm + residual_norm);
-  const double target = std::max(10 * c.opts.linear_tol * residual_norm, allowance);
+  // norms of an update are formed on the device and read with the status words
+  // that a phase fetches anyway
+  launch_wnorm2(c, c.u, c.nu, c.mtab_dg, c.m, DS_U);
+  double allowance = 0., target = 0.;
+  const auto set_target = [&] {
+    allowance = 128 * eps * (std::sqrt(c.hscal[DS_U]) + old_norm + residual_norm);
+    target = std::max(10 * c.opts.linear_tol * residual_norm, allowance);
+  };
+  const auto part_seconds = [&](int a, int b) {
+    float ms = 0.f;
+    EG_CUDA(cudaEventElapsedTime(&ms, c.ev_part[a], c.ev_part[b]));
+    return 1e-3 * ms;
+  };
   double er_norm = 0.;
   LinearOut lr;
   int total_count = 0;
   if (form == EG_FORM_DG) {
-    // Jacobians are evaluated from the Newton state inside every action.
     launch_axpby(c, c.nu, -1., c.r, 0., c.r, c.tmp_body);
-    linear_solve(c, EG_FORM_DG, c.tmp_body, c.du, c.er, true, c.opts.linear_tol, lr);
+    linear_solve(c, EG_FORM_DG, c.tmp_body, c.du, c.er, true, c.opts.linear_tol, lr, residual_norm);
     total_count = lr.count;
     s.assembly_s = lr.assembly;
     s.setup_s = lr.setup;
     s.solve_s = lr.solve;
     const double v0 = now_s();
     er_norm = cell_norm(c, c.er);
+    set_target();
     s.validation_s = now_s() - v0;
   } else {
+    // with block Jacobi, the factor and the norm of the right-hand side follow
+    // the condensation before the host looks at either
+    const bool ahead = c.opts.precond == EG_PC_BLOCK_JACOBI && c.opts.assembly != EG_ASSEMBLY_FULL &&
+                       c.opts.solver == EG_SOLVER_GMRES;
+    const auto follow = [&] {
+      if (!ahead) return;
+      EG_CUDA(cudaEventRecord(c.ev_part[1], c.stream));
+      launch_wnorm2(c, c.rhs, c.nl, c.mtab_hdg, 2 * c.t, DS_RHS);
+      launch_schur_jacobi(c, true);
+      EG_CUDA(cudaEventRecord(c.ev_part[2], c.stream));
+    };
     const double c0 = now_s();
-    condense(c, c.u, c.r);
-    s.condensation_s = now_s() - c0;
+    condense_launch(c, c.u, c.r);
+    follow();
+    c.fetch_status();
+    if (condense_finish(c, c.u, c.r) && ahead) {
+      follow();
+      c.check_device_error();
+    }
+    const double setup = ahead ? part_seconds(1, 2) : 0.;
+    s.setup_s = setup;
+    s.condensation_s = now_s() - c0 - setup;
+    const double rhs_norm = ahead ? std::sqrt(c.hscal[DS_RHS]) : -1.;
     double tol = c.opts.linear_tol;
     bool valid = false;
     for (int attempt = 0; attempt < 4; ++attempt) {
       LinearOut a;
-      linear_solve(c, EG_FORM_HDG, c.rhs, c.lam, c.tmp_trace, attempt == 0, tol, a);
+      linear_solve(c, EG_FORM_HDG, c.rhs, c.lam, c.tmp_trace, attempt == 0, tol, a, rhs_norm, ahead);
       total_count += a.count;
       s.assembly_s += a.assembly;
       s.setup_s += a.setup;
       s.solve_s += a.solve;
       lr.residual = a.residual;
       const double r0 = now_s();
+      EG_CUDA(cudaEventRecord(c.ev_part[0], c.stream));
       launch_recover(c, c.lam, c.du);
-      c.sync();
-      s.recovery_s += now_s() - r0;
-      const double v0 = now_s();
+      EG_CUDA(cudaEventRecord(c.ev_part[3], c.stream));
       launch_recovered_residual(c, c.tmp_trace, c.er);
-      er_norm = cell_norm(c, c.er);
-      s.validation_s += now_s() - v0;
+      launch_wnorm2(c, c.er, c.nu, c.mtab_dg, c.m, DS_ER);
+      c.fetch_status();
+      er_norm = std::sqrt(c.hscal[DS_ER]);
+      set_target();
+      const double recovery = part_seconds(0, 3);
+      s.recovery_s += recovery;
+      s.validation_s += now_s() - r0 - recovery;
       s.attempts = attempt + 1;
       valid = er_norm <= target;
       if (valid) break;
@@ -411,16 +458,17 @@ void newton_update(Ctx &c, double residual_norm, double old_norm, eg_update_stat
   double damping = 1.;
   bool accept = false;
   for (int back = 0; back < 30; ++back) {
+    // the residual of the trial is formed before its admissibility is known:
+    // one round trip instead of two
     launch_axpby(c, c.nu, 1., c.u, damping, c.du, c.trial);
     launch_admissible(c, c.trial);
-    EG_CUDA(cudaMemcpyAsync(c.herr + 1, c.derr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.sync();
-    if (c.herr[1]) {
-      launch_residual(c, c.trial, c.old, c.trial_r);
-      if (cell_norm(c, c.trial_r) <= (1 - 1e-4 * damping) * residual_norm + allowance) {
-        accept = true;
-        break;
-      }
+    launch_residual(c, c.trial, c.old, c.trial_r);
+    launch_wnorm2(c, c.trial_r, c.nu, c.mtab_dg, c.m, DS_NORM);
+    EG_CUDA(cudaEventRecord(c.ev1, c.stream));
+    c.fetch_status();
+    if (c.herr[1] && std::sqrt(c.hscal[DS_NORM]) <= (1 - 1e-4 * damping) * residual_norm + allowance) {
+      accept = true;
+      break;
     }
     damping *= .5;
   }
@@ -431,8 +479,6 @@ void newton_update(Ctx &c, double residual_norm, double old_norm, eg_update_stat
   s.line_search_s = now_s() - ls0;
   s.damping = damping;
   s.residual_norm = residual_norm;
-  EG_CUDA(cudaEventRecord(c.ev1, c.stream));
-  c.sync();
   float ms = 0.f;
   EG_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
   c.update_timer_open = false;
@@ -619,6 +665,7 @@ int eg_create(const eg_desc *d, const eg_opts *o, eg_ctx **out) {
     EG_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     EG_CUDA(cudaEventCreate(&c.ev0));
     EG_CUDA(cudaEventCreate(&c.ev1));
+    for (cudaEvent_t &e : c.ev_part) EG_CUDA(cudaEventCreate(&e));
     const int q = c.q;
     c.tab = c.alloc_n<double>(eg::tab_size(q));
     c.mtab_dg = c.alloc_n<double>(c.p);
@@ -634,17 +681,17 @@ int eg_create(const eg_desc *d, const eg_opts *o, eg_ctx **out) {
     }
     c.D = c.alloc_n<double>(c.nl);
     EG_CUDA(cudaMemsetAsync(c.D, 0, sizeof(double) * c.nl, c.stream));
-    c.derr = c.alloc_n<int>(4);
-    EG_CUDA(cudaMemsetAsync(c.derr, 0, 4 * sizeof(int), c.stream));
-    c.dscal = c.alloc_n<double>(eg::DS_COUNT);
-    EG_CUDA(cudaMemsetAsync(c.dscal, 0, eg::DS_COUNT * sizeof(double), c.stream));
+    constexpr size_t status_bytes = 4 * sizeof(int) + eg::DS_COUNT * sizeof(double);
+    c.derr = static_cast<int *>(c.alloc(status_bytes));
+    c.dscal = reinterpret_cast<double *>(c.derr + 4);
+    EG_CUDA(cudaMemsetAsync(c.derr, 0, status_bytes, c.stream));
     c.counter = c.alloc_n<unsigned>(1);
     EG_CUDA(cudaMemsetAsync(c.counter, 0, sizeof(unsigned), c.stream));
     c.partials = c.alloc_n<double>((size_t)eg::kRedBlocks * (eg::kMaxRestart + 1));
     c.ctl = c.alloc_n<eg::GmresCtl>(1);
     EG_CUDA(cudaMallocHost(&c.hctl, sizeof(eg::GmresCtl)));
-    EG_CUDA(cudaMallocHost(&c.hscal, sizeof(double) * eg::DS_COUNT));
-    EG_CUDA(cudaMallocHost(&c.herr, sizeof(int) * 4));
+    EG_CUDA(cudaMallocHost(&c.herr, status_bytes));
+    c.hscal = reinterpret_cast<double *>(c.herr + 4);
     if (o->form == EG_FORM_HDG) c.ensure_hdg();
     c.sync();
   });
@@ -669,10 +716,11 @@ void eg_destroy(eg_ctx *ctx) {
   for (cudaEvent_t e : c.prof.pool) cudaEventDestroy(e);
   for (void *p : c.allocations) cudaFree(p);
   if (c.hctl) cudaFreeHost(c.hctl);
-  if (c.hscal) cudaFreeHost(c.hscal);
   if (c.herr) cudaFreeHost(c.herr);
   if (c.ev0) cudaEventDestroy(c.ev0);
   if (c.ev1) cudaEventDestroy(c.ev1);
+  for (cudaEvent_t e : c.ev_part)
+    if (e) cudaEventDestroy(e);
   if (c.stream) cudaStreamDestroy(c.stream);
   delete ctx;
 }
@@ -769,17 +817,16 @@ int eg_freeze(eg_ctx *ctx, double stage_dt, int check_admissible, double *wave_r
   return guard(ctx, [&] {
     Ctx &c = ctx->c;
     eg::launch_freeze(c, c.u, check_admissible != 0);
-    c.check_device_error();
-    eg::launch_copy(c, c.nu, c.u, c.old);
+    eg::launch_keep_old(c, check_admissible != 0);
+    c.fetch_status();
+    if (check_admissible && !c.herr[1]) {
+      c.herr[0] = 0;
+      eg::fail(EG_ERR_INADMISSIBLE, "Old state is inadmissible; refine mesh");
+    }
+    c.raise_device_error();
     c.geo.dt = stage_dt;
     c.residual_ready = false;
-    if (wave_rate) {
-      EG_CUDA(cudaMemcpyAsync(c.hscal + eg::DS_WAVE, c.dscal + eg::DS_WAVE, sizeof(double),
-                              cudaMemcpyDeviceToHost, c.stream));
-      c.sync();
-      *wave_rate = c.hscal[eg::DS_WAVE] / std::min(c.desc.hx, c.desc.hy);
-    }
-    c.sync();
+    if (wave_rate) *wave_rate = c.hscal[eg::DS_WAVE] / std::min(c.desc.hx, c.desc.hy);
   });
 }
 
@@ -818,9 +865,8 @@ int eg_admissible(eg_ctx *ctx, int slot, int *ok) {
     const double *x = eg::slot_ptr(c, slot, count);
     if ((int)count != c.nu) eg::fail(EG_ERR_INVALID, "size mismatch");
     eg::launch_admissible(c, x);
-    EG_CUDA(cudaMemcpyAsync(c.herr + 1, c.derr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.sync();
-    *ok = c.herr[1];
+    c.fetch_status();
+    *ok = c.herr[1] != 0;
   });
 }
 

@@ -27,9 +27,10 @@ __global__ void __launch_bounds__(256) freeze_kernel(Geo g, const double *__rest
                                                      const double *__restrict__ u, double *fa,
                                                      double *fb, double *flw, double *frw,
                                                      double *fpen, double *D, int *err,
-                                                     unsigned long long *wave) {
+                                                     unsigned long long *wave, const int *admissible) {
   __shared__ STab<Q> st;
   __shared__ double red[256];
+  if (admissible != nullptr && *admissible == 0) return;  // refused: the frozen data stay
   load_tables<Q>(st, tab);
   __syncthreads();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -532,25 +533,33 @@ __global__ void __launch_bounds__(256)
 static Frozen frozen_of(Ctx &c) { return Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}; }
 
 void launch_freeze(Ctx &c, const double *u, bool check_admissible) {
-  if (check_admissible) {
-    launch_admissible(c, u);
-    EG_CUDA(cudaMemcpyAsync(c.herr + 1, c.derr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.sync();
-    if (!c.herr[1]) fail(EG_ERR_INADMISSIBLE, "Old state is inadmissible; refine mesh");
-  }
+  if (check_admissible) launch_admissible(c, u);
   EG_CUDA(cudaMemsetAsync(c.dscal + DS_WAVE, 0, sizeof(double), c.stream));
   const int total = c.nf * c.q;
   const int blocks = (total + 255) / 256;
   ProfScope ps(c, EG_K_FREEZE, 1);
   EG_DISPATCH_Q(c.q, freeze_kernel<Q><<<blocks, 256, 0, c.stream>>>(
                          c.geo, c.tab, u, c.fa, c.fbb, c.flw, c.frw, c.fpen, c.D, c.derr,
-                         reinterpret_cast<unsigned long long *>(c.dscal + DS_WAVE)));
+                         reinterpret_cast<unsigned long long *>(c.dscal + DS_WAVE),
+                         check_admissible ? c.derr + 1 : nullptr));
+  EG_CUDA(cudaGetLastError());
+}
+
+__global__ void __launch_bounds__(256) keep_old_kernel(int n2, const double2 *__restrict__ u, double2 *__restrict__ old,
+                                                       const int *err, bool checked) {
+  if (err[0] != 0 || (checked && err[1] == 0)) return;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += gridDim.x * blockDim.x) old[i] = u[i];
+}
+void launch_keep_old(Ctx &c, bool checked) {
+  const int n2 = c.nu / 2;  // nu is a multiple of 4
+  ProfScope ps(c, EG_K_VECTOR, 1);
+  keep_old_kernel<<<std::min((n2 + 255) / 256, 148 * 16), 256, 0, c.stream>>>(
+      n2, reinterpret_cast<const double2 *>(c.u), reinterpret_cast<double2 *>(c.old), c.derr, checked);
   EG_CUDA(cudaGetLastError());
 }
 
 void launch_admissible(Ctx &c, const double *u) {
-  const int one = 1;
-  EG_CUDA(cudaMemcpyAsync(c.derr + 1, &one, sizeof(int), cudaMemcpyHostToDevice, c.stream));
+  EG_CUDA(cudaMemsetAsync(c.derr + 1, 1, sizeof(int), c.stream));  // any nonzero word
   ProfScope ps(c, EG_K_ADMISSIBLE, 1);
   EG_DISPATCH_Q(c.q, {
     using C = CellCfg<Q>;

@@ -180,6 +180,7 @@ void launch_dg_inverse(Ctx &c, const double *u) {
                          count, c.derr)));
   EG_CUDA(cudaGetLastError());
   EG_CUDA(cudaMemsetAsync(c.derr + 3, 0, sizeof(int), c.stream));
+  c.check_device_error();
 }
 
 void launch_dg_inverse_apply(Ctx &c, const double *b, double *x) {

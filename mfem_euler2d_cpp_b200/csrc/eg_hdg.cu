@@ -650,7 +650,7 @@ static void condense_redo(Ctx &c, const double *u, const double *r, int count) {
   launch_condensed_rhs(c);
 }
 
-void condense(Ctx &c, const double *u, const double *r) {
+void condense_launch(Ctx &c, const double *u, const double *r) {
   c.ensure_hdg();
   {
     ProfScope ps(c, EG_K_CONDENSE, 2);
@@ -667,11 +667,25 @@ void condense(Ctx &c, const double *u, const double *r) {
     launch_condensed_rhs(c);
   }
   c.condensed = true;
-  c.check_device_error();
-  if (const int count = c.herr[3]) {
-    condense_redo(c, u, r, count);
-    c.check_device_error();
+}
+
+bool condense_finish(Ctx &c, const double *u, const double *r) {
+  const int count = c.herr[3];
+  if (count == 0) {
+    c.raise_device_error();
+    return false;
   }
+  // an error raised so far is of work on the unfinished system
+  EG_CUDA(cudaMemsetAsync(c.derr, 0, sizeof(int), c.stream));
+  condense_redo(c, u, r, count);
+  c.check_device_error();
+  return true;
+}
+
+void condense(Ctx &c, const double *u, const double *r) {
+  condense_launch(c, u, r);
+  c.fetch_status();
+  condense_finish(c, u, r);
 }
 
 void launch_schur_apply(Ctx &c, const double *v, double *y) {

@@ -45,7 +45,9 @@ enum DScal : int {
   DS_NORM = 0,       // generic reduction result
   DS_NORM2 = 1,
   DS_WAVE = 2,       // max HLL speed bits (as unsigned long long)
-  DS_ADMISSIBLE = 3, // 1.0 when admissible
+  DS_U = 3,          // Newton update: norms of the state, of the Schur
+  DS_RHS = 4,        // right-hand side and of the recovered residual, read
+  DS_ER = 5,         // together with the error words
   DS_COUNT = 8
 };
 
@@ -221,14 +223,16 @@ struct Ctx {
   const int *skip = nullptr;
   double *partials = nullptr;  // kRedBlocks * (kMaxRestart+1)
   unsigned *counter = nullptr;
-  // error word (derr[0]) and admissibility flag (derr[1])
+  // status words: error (derr[0]), admissibility (derr[1], nonzero when
+  // admissible), context lost (derr[2]), cells to solve again (derr[3]); the
+  // scalars follow them, so that one copy brings both to the host
   int *derr = nullptr;
   double *dscal = nullptr;
   double *field_partial = nullptr;  // per-cell partials of the diagnostics (4n) and their sum (4)
   double *hscal = nullptr;  // pinned mirror of dscal
   int *herr = nullptr;      // pinned
   // events for per-update device timing
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_part[4] = {};
   double last_residual_s = 0.;
   bool update_timer_open = false;
 
@@ -262,13 +266,21 @@ struct Ctx {
   void ensure_pc_dg();
   void ensure_pc_hdg();
   void sync();
-  void check_device_error();
+  // one copy of the status words and scalars, and the stream synchronised
+  void fetch_status();
+  void check_device_error();  // fetch_status, and an error raised
+  void raise_device_error();  // of the status fetched last
   void prof_resolve();
 };
 
 // ---- launchers (eg_cell.cu) ----
+// check_admissible: a state that is not admissible leaves the frozen data as
+// they were (the caller reads derr[1])
 void launch_freeze(Ctx &c, const double *u, bool check_admissible);
-void launch_admissible(Ctx &c, const double *u);  // writes dscal[DS_ADMISSIBLE]
+// old <- u, unless the last launch_freeze met an error or (checked) an
+// inadmissible state
+void launch_keep_old(Ctx &c, bool checked);
+void launch_admissible(Ctx &c, const double *u);  // sets derr[1]
 void launch_residual(Ctx &c, const double *u, const double *old, double *r);
 void launch_dg_apply(Ctx &c, const double *u, const double *x, double *y);  // Jacobians recomputed
 // PartialDGOperator::Refresh at state u, then the cached action (Mult)
@@ -287,6 +299,11 @@ void launch_dg_inverse_apply(Ctx &c, const double *b, double *x);
 // condensation of every cell at state u with residual r; synchronises and
 // raises a singular cell
 void condense(Ctx &c, const double *u, const double *r);
+// the same in two parts: the launches, then a look at the status fetched after
+// them; true when cells had to be solved again (what was launched on the
+// condensed system in between is to be repeated)
+void condense_launch(Ctx &c, const double *u, const double *r);
+bool condense_finish(Ctx &c, const double *u, const double *r);
 // k >= 6: one thread-block cluster per cell (eg_cluster.cu); the second writes
 // the explicit DG block-Jacobi inverses to pc_dg
 void launch_condense_cluster(Ctx &c, const double *u, const double *r);

@@ -428,16 +428,12 @@ void launch_wnorm2(Ctx &c, const double *x, int N, const double *mtab, int perio
 template <class T>
 double wnorm_t(Ctx &c, const T *x, int N, const double *mtab, int period) {
   launch_wnorm2_t(c, x, N, mtab, period, DS_NORM);
-  EG_CUDA(cudaMemcpyAsync(c.hscal + DS_NORM, c.dscal + DS_NORM, sizeof(double),
-                          cudaMemcpyDeviceToHost, c.stream));
-  c.sync();
+  c.fetch_status();
   return std::sqrt(c.hscal[DS_NORM]);
 }
 double wnorm(Ctx &c, const double *x, int N, const double *mtab, int period) {
   launch_wnorm2(c, x, N, mtab, period, DS_NORM);
-  EG_CUDA(cudaMemcpyAsync(c.hscal + DS_NORM, c.dscal + DS_NORM, sizeof(double),
-                          cudaMemcpyDeviceToHost, c.stream));
-  c.sync();
+  c.fetch_status();
   return std::sqrt(c.hscal[DS_NORM]);
 }
 double cell_norm(Ctx &c, const double *x) { return wnorm(c, x, c.nu, c.mtab_dg, c.m); }

@@ -81,8 +81,7 @@ struct Stepper {
     }
     field_initial(c, c.u);  // Problem::Initial on the device
     launch_admissible(c, c.u);
-    EG_CUDA(cudaMemcpyAsync(c.herr + 1, c.derr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.sync();
+    c.fetch_status();
     if (!c.herr[1]) fail(EG_ERR_INITIAL, "Initial projection not positive; refine mesh");
     field_integral(c, c.u, initial_integral);
     stage_count = ro.integrator == 1 ? 1 : 4;
@@ -103,9 +102,6 @@ struct Stepper {
   void begin_step() {
     launch_copy(c, c.nu, c.u, step_state);
     freeze_at_u(ro.dt);
-    EG_CUDA(cudaMemcpyAsync(c.hscal + DS_WAVE, c.dscal + DS_WAVE, sizeof(double), cudaMemcpyDeviceToHost,
-                            c.stream));
-    c.sync();
     rate = c.hscal[DS_WAVE] / std::min(c.desc.hx, c.desc.hy);
     dt = ro.cfl > 0 ? ro.cfl / rate : ro.dt;
     if (ro.steps < 0) {
@@ -152,8 +148,7 @@ struct Stepper {
       for (int s = 0; s < 4; ++s) grid_add(dt * kB[s], slope[s], c.u);
       c.residual_ready = false;
       launch_admissible(c, c.u);
-      EG_CUDA(cudaMemcpyAsync(c.herr + 1, c.derr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-      c.sync();
+      c.fetch_status();
       if (!c.herr[1]) fail(EG_ERR_DIRK_INADMISSIBLE, "SSP-DIRK3 step produced an inadmissible state");
     }
     time = ro.steps < 0 && final_step ? ro.end : time + dt;
