@@ -62,41 +62,35 @@ __device__ __forceinline__ unsigned long long global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// Waits are bounded in time: a wait that has polled for more than limit_ns
-// nanoseconds (read every 64 polls from the global timer) gives up.
+// Waits are bounded in time. A poll reads the awaited word only: the abort word
+// and the global timer, each a round trip to L2 (about 700 cycles), are looked
+// at every 32 or 256 polls.
+constexpr unsigned kCheckGlobal = 31, kCheckLocal = 255;
+__device__ __forceinline__ bool out_of_time(unsigned long long &t0, int *abort, int *err, unsigned long long limit_ns) {
+  if (ld_volatile(abort)) return true;
+  const unsigned long long now = global_ns();
+  if (t0 == 0) t0 = now;
+  if (now - t0 <= limit_ns) return false;
+  give_up(abort, err);
+  return true;
+}
 // Bounded wait until *p >= target (another CTA's progress).
 __device__ bool wait_progress(const unsigned long long *p, unsigned long long target, int *abort, int *err,
                               unsigned long long limit_ns) {
   unsigned long long t0 = 0;
-  for (unsigned it = 0;; ++it) {
+  for (unsigned it = 1;; ++it) {
     if (ld_acquire(p) >= target) return true;
-    if (ld_volatile(abort)) return false;
-    if (it >= 16) __nanosleep(64);
-    if ((it & 63u) == 0) {
-      const unsigned long long now = global_ns();
-      if (it == 0) t0 = now;
-      else if (now - t0 > limit_ns) break;
-    }
+    if ((it & kCheckGlobal) == 0 && out_of_time(t0, abort, err, limit_ns)) return false;
   }
-  give_up(abort, err);
-  return false;
 }
 // Bounded wait until the CTA's own published row count reaches target.
 __device__ bool wait_local(const volatile unsigned *count, unsigned target, int *abort, int *err,
                            unsigned long long limit_ns) {
   unsigned long long t0 = 0;
-  for (unsigned it = 0;; ++it) {
+  for (unsigned it = 1;; ++it) {
     if (*count >= target) return true;
-    if (ld_volatile(abort)) return false;
-    if (it >= 16) __nanosleep(32);
-    if ((it & 63u) == 0) {
-      const unsigned long long now = global_ns();
-      if (it == 0) t0 = now;
-      else if (now - t0 > limit_ns) break;
-    }
+    if ((it & kCheckLocal) == 0 && out_of_time(t0, abort, err, limit_ns)) return false;
   }
-  give_up(abort, err);
-  return false;
 }
 // The progress value a wait needs: `starve` (a test setting) asks for one no
 // CTA ever publishes, so every wait on another CTA runs out.
@@ -133,6 +127,8 @@ struct SweepArgs {
   int staged;        // stage up to kStageBlocks blocks per row in shared memory
   unsigned long long limit_ns;  // bound of every wait
   int starve;        // test setting: waits on other CTAs can never be met
+  uint4 *slots;      // small blocks: the rows' values for other CTAs
+  unsigned epoch;
 };
 
 // FixedBlockILU::Mult (src/block_ilu.cpp:88-109). Forward: w_i = b_i -
@@ -223,9 +219,13 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_kernel(SweepArgs a) {
           for (int s = 0; s < S; ++s) {
             const int r = lane + 32 * s;
             if (r < B) {
-              double t = acc[s];
-              for (int cc = 0; cc < B; ++cc) t -= A[(size_t)cc * B + r] * vb[cc];
-              acc[s] = t;
+              // four partial sums: B is a multiple of 4, and one chain of B
+              // dependent products would be most of a row's time
+              double t[4] = {acc[s], 0., 0., 0.};
+              for (int cc = 0; cc < B; cc += 4)
+#pragma unroll
+                for (int k4 = 0; k4 < 4; ++k4) t[k4] -= A[(size_t)(cc + k4) * B + r] * vb[cc + k4];
+              acc[s] = (t[0] + t[1]) + (t[2] + t[3]);
             }
           }
           __syncwarp();
@@ -245,9 +245,11 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_kernel(SweepArgs a) {
       for (int s = 0; s < S; ++s) {
         const int r = lane + 32 * s;
         if (r < B) {
-          double t = 0.;
-          for (int cc = 0; cc < B; ++cc) t += Di[(size_t)cc * B + r] * vb[cc];
-          acc[s] = t;
+          double t[4] = {0., 0., 0., 0.};
+          for (int cc = 0; cc < B; cc += 4)
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4) t[k4] += Di[(size_t)(cc + k4) * B + r] * vb[cc + k4];
+          acc[s] = (t[0] + t[1]) + (t[2] + t[3]);
         }
       }
       __syncwarp();
@@ -275,9 +277,206 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_kernel(SweepArgs a) {
   }
 }
 
+// A row's values for other CTAs travel as self-validating words: each 8-byte
+// half of a slot carries 32 bits of a value and the sweep's epoch, so a reader
+// polls the values themselves (one trip through L2) instead of a counter that
+// is released behind a fence and then the values (three).
+__device__ __forceinline__ void put_slot(uint4 *p, double v, unsigned ep) {
+  asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"((unsigned)__double2loint(v)),
+               "r"(ep), "r"((unsigned)__double2hiint(v)), "r"(ep)
+               : "memory");
+}
+__device__ __forceinline__ bool get_slot(const uint4 *p, unsigned ep, double &v) {
+  unsigned lo, e0, hi, e1;
+  asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(lo), "=r"(e0), "=r"(hi), "=r"(e1)
+               : "l"(p)
+               : "memory");
+  v = __hiloint2double((int)hi, (int)lo);
+  return e0 == ep && e1 == ep;
+}
+
+// The sweep for blocks of at most kStageMaxB (every HDG degree, DG up to k =
+// 2), the block size known at compile time. What bounds it is the chain of
+// dependent rows: a grid row of faces starts three to five rows behind its
+// neighbour, so a sweep is ny times (a few rows + one hand-over between CTAs).
+// A row's products are four partial sums each, unrolled; its neighbours' rows
+// in other CTAs are polled together and folded in before its own CTA's.
+// 48x48 Q4, forward and backward sweep: 1190 us with the counters and run-time
+// block sizes of the kernel above, see the launch table in the driver below.
+template <int B, bool BACK>
+__global__ void __launch_bounds__(256, 1) ilu_sweep_small_kernel(SweepArgs a) {
+  constexpr int S = (B + 31) / 32, BB = B * B;
+  extern __shared__ __align__(128) double smem[];
+  __shared__ unsigned done_local;
+  __shared__ __align__(8) unsigned long long bars[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int g = blockIdx.x;
+  const int p0 = a.slot_ptr[g], nslots = a.slot_ptr[g + 1] - p0;
+  double *stage = smem + (size_t)warp * kStageBlocks * BB;
+  double *vb = smem + (size_t)W * kStageBlocks * BB + (size_t)warp * kMaxDeps * B;
+  double *ring = smem + (size_t)W * (kStageBlocks * BB + kMaxDeps * B);
+  if (threadIdx.x == 0) done_local = 0;
+  if (lane == 0) mbar_init(&bars[warp]);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncthreads();
+  volatile unsigned *dl = &done_local;
+  unsigned phase = 0;
+  int4 nm = make_int4(0, 0, 0, 0);
+  int2 nd[kMaxDeps];
+  auto fetch = [&](int slot) {
+    if (slot < nslots) {
+      nm = a.meta[p0 + slot];
+#pragma unroll
+      for (int k = 0; k < kMaxDeps; ++k) nd[k] = a.deps[(size_t)(p0 + slot) * kMaxDeps + k];
+    }
+  };
+  fetch(warp);
+  for (int slot = warp; slot < nslots; slot += W) {
+    const int i = nm.x, e0 = nm.y, ne = nm.z;
+    int2 dep[kMaxDeps];
+#pragma unroll
+    for (int k = 0; k < kMaxDeps; ++k) dep[k] = nd[k];
+    const int nst = min(ne, BACK ? kStageBlocks - 1 : kStageBlocks);
+    const bool copy = nst > 0 || BACK;
+    if (copy && lane == 0) {
+      const unsigned bytes = (unsigned)(sizeof(double) * BB * (nst + (BACK ? 1 : 0)));
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mbar_expect(&bars[warp], bytes);
+      if (nst) bulk_load(stage, a.data + (size_t)e0 * BB, (unsigned)(sizeof(double) * BB * nst), &bars[warp]);
+      if (BACK)
+        bulk_load(stage + (size_t)nst * BB, a.dinv + (size_t)i * BB, (unsigned)(sizeof(double) * BB), &bars[warp]);
+    }
+    fetch(slot + W);  // the next row's schedule is in flight during this row
+    double acc[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      const int r = lane + 32 * s;
+      acc[s] = r < B ? __ldcg(a.in + (size_t)i * B + r) : 0.;
+    }
+    // values of the rows other CTAs own, all polled together
+    bool ok = true;
+    unsigned missing = 0u;  // one bit per dependency still to come (per lane)
+#pragma unroll
+    for (int k = 0; k < kMaxDeps; ++k)
+      if (k < ne && (dep[k].x >> kOwnerShift) != g) missing |= 1u << k;
+    {
+      const unsigned want = a.starve ? a.epoch + 1u : a.epoch;
+      unsigned long long t0 = 0;
+      for (unsigned it = 1; __any_sync(0xffffffffu, missing != 0u); ++it) {
+#pragma unroll
+        for (int k = 0; k < kMaxDeps; ++k)
+          if ((missing >> k) & 1u) {
+            bool got = true;
+            double v[S];
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+              const int r = lane + 32 * s;
+              v[s] = 0.;
+              if (r < B) got = get_slot(a.slots + (size_t)dep[k].y * B + r, want, v[s]) && got;
+            }
+            if (got) {
+              missing &= ~(1u << k);
+#pragma unroll
+              for (int s = 0; s < S; ++s)
+                if (lane + 32 * s < B) vb[k * B + lane + 32 * s] = v[s];
+            }
+          }
+        if ((it & kCheckGlobal) == 0) {
+          int late = 0;
+          if (lane == 0) late = out_of_time(t0, a.abort, a.err, a.limit_ns);
+          if (__shfl_sync(0xffffffffu, late, 0)) {
+            ok = false;
+            break;
+          }
+        }
+      }
+    }
+    if (copy) {
+      if (!mbar_wait(&bars[warp], phase, kCopySpinLimit)) {
+        give_up(a.abort, a.err);
+        // let the copy land before the CTA can exit; if even the longer drain
+        // bound runs out, the copy may still write this CTA's shared memory:
+        // err[2] tells the host that the context can no longer be trusted
+        if (!mbar_wait(&bars[warp], phase, kDrainSpinLimit) && lane == 0) atomicExch(a.err + 2, 1);
+        return;
+      }
+      phase ^= 1u;
+    }
+    if (!ok) return;
+    __syncwarp();
+    const auto product = [&](const double *A, const double *v, double sign) {
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        const int r = lane + 32 * s;
+        if (r < B) {
+          double t[4] = {0., 0., 0., 0.};
+#pragma unroll
+          for (int cc = 0; cc < B; cc += 4)
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4) t[k4] = fma(A[(cc + k4) * B + r], v[cc + k4], t[k4]);
+          acc[s] = fma(sign, (t[0] + t[1]) + (t[2] + t[3]), acc[s]);
+        }
+      }
+    };
+#pragma unroll
+    for (int k = 0; k < kMaxDeps; ++k)
+      if (k < ne && (dep[k].x >> kOwnerShift) != g)
+        product(k < nst ? stage + (size_t)k * BB : a.data + (size_t)(e0 + k) * BB, vb + k * B, -1.);
+    // the CTA's own rows, the ones finished first in front
+#pragma unroll
+    for (int k0 = 0; k0 < kMaxDeps; ++k0) {
+      const int k = BACK ? kMaxDeps - 1 - k0 : k0;
+      if (k < ne && (dep[k].x >> kOwnerShift) == g && ok) {
+        const int js = dep[k].x & kSlotMask;
+        ok = wait_local(dl, (unsigned)js + 1, a.abort, a.err, a.limit_ns);
+        if (ok) {
+          __threadfence_block();
+          const double *v = ring + (size_t)(js & (a.ring - 1)) * B;
+          if (slot - js > a.ring - W) {  // gone from the ring
+            for (int r = lane; r < B; r += 32) vb[k * B + r] = __ldcg(a.out + (size_t)dep[k].y * B + r);
+            __syncwarp();
+            v = vb + k * B;
+          }
+          product(k < nst ? stage + (size_t)k * BB : a.data + (size_t)(e0 + k) * BB, v, -1.);
+        }
+      }
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) return;
+    if (BACK) {
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+        if (lane + 32 * s < B) vb[lane + 32 * s] = acc[s];
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < S; ++s) acc[s] = 0.;
+      product(stage + (size_t)nst * BB, vb, 1.);
+    }
+    double *rs = ring + (size_t)(slot & (a.ring - 1)) * B;
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      const int r = lane + 32 * s;
+      if (r < B) {
+        rs[r] = acc[s];
+        put_slot(a.slots + (size_t)i * B + r, acc[s], a.epoch);
+        a.out[(size_t)i * B + r] = acc[s];
+      }
+    }
+    __threadfence_block();
+    __syncwarp();
+    int pub = 1;
+    if (lane == 0) {
+      pub = wait_local(dl, (unsigned)slot, a.abort, a.err, a.limit_ns);  // rows are published in order
+      if (pub) *dl = (unsigned)slot + 1;
+    }
+    if (!__shfl_sync(0xffffffffu, pub, 0)) return;
+  }
+}
+
 // ----------------------------------------------------------- factor kernel
 struct FactorArgs {
-  int B, maxrow, maxupd;
+  int B, maxrow, maxupd, maxl, maxtot;
   const int *slot_ptr;
   const int4 *meta;   // forward schedule: (row, first lower entry, lower count)
   const int2 *deps;
@@ -385,6 +584,117 @@ __global__ void __launch_bounds__(256, 1) ilu_factor_kernel(FactorArgs a) {
     for (int o = threadIdx.x; o < BB; o += blockDim.x) Di[o] = Inv[o];
     if (SMEM)
       for (int o = threadIdx.x; o < (re - rb) * BB; o += blockDim.x) a.data[(size_t)rb * BB + o] = rowblk[o];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) publish_max(a.progress + g, a.tag | (unsigned long long)(slot + 1));
+  }
+}
+
+// Factor for blocks of at most 32 (every HDG degree below 8): the arithmetic
+// of ilu_factor_kernel with the block size known at compile time. A row's
+// blocks are read before its neighbours are waited for, all blocks of the
+// neighbours (inverse diagonals and retained U) in one round, and the diagonal
+// block is inverted by one warp in registers, a row per lane: Gauss-Jordan in
+// place with row pivoting, no barrier in its steps. One CTA per row as there;
+// the chain of rows bounds it, so what counts is the latency of a row.
+// 48x48 Q4: 16.3 ms with the kernel above, see the driver below.
+template <int B>
+__global__ void __launch_bounds__(512, 1) ilu_factor_small_kernel(FactorArgs a) {
+  constexpr int BB = B * B;
+  extern __shared__ __align__(16) double fsm[];
+  __shared__ int stop;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = blockIdx.x, p0 = a.slot_ptr[g], nslots = a.slot_ptr[g + 1] - p0;
+  double *rowblk = fsm;                              // the row's blocks (maxrow)
+  double *Dk = rowblk + (size_t)a.maxrow * BB;       // U_kk^{-1} of the lower neighbours (maxl)
+  double *Ub = Dk + (size_t)a.maxl * BB;             // their retained U_kj (maxtot)
+  double *Lt = Ub + (size_t)a.maxtot * BB;
+  for (int slot = 0; slot < nslots; ++slot) {
+    const int4 m = a.meta[p0 + slot];
+    const int i = m.x, nl = m.z, rb = a.row[i], re = a.row[i + 1], di = a.diag[i];
+    const int u0 = a.upd_ptr[rb], ntot = a.upd_ptr[di] - u0;
+    for (int o = threadIdx.x; o < (re - rb) * BB; o += blockDim.x) rowblk[o] = a.data[(size_t)rb * BB + o];
+    if (threadIdx.x == 0) {
+      int ok = 1;
+      for (int k = 0; k < nl && ok; ++k) {
+        const int2 d = a.deps[(size_t)(p0 + slot) * kMaxDeps + k];
+        const int owner = d.x >> kOwnerShift, js = d.x & kSlotMask;
+        if (owner != g)
+          ok = wait_progress(a.progress + owner, need(a.tag, js, a.starve), a.abort, a.err, a.limit_ns);
+      }
+      stop = !ok;
+    }
+    __syncthreads();
+    if (stop) return;
+    for (int o = threadIdx.x; o < (nl + ntot) * BB; o += blockDim.x) {
+      const int blk = o / BB, r = o % BB;
+      Dk[blk < nl ? o : (a.maxl - nl) * BB + o] =
+          blk < nl ? __ldcg(a.dinv + (size_t)a.deps[(size_t)(p0 + slot) * kMaxDeps + blk].y * BB + r)
+                   : __ldcg(a.data + (size_t)a.upd[2 * (u0 + blk - nl) + 1] * BB + r);
+    }
+    __syncthreads();
+    const auto dot = [](const double *A, const double *C) {  // row of A (stride B) times a column of C
+      double t[4] = {0., 0., 0., 0.};
+#pragma unroll
+      for (int s = 0; s < B; s += 4)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) t[k] = fma(A[(s + k) * B], C[s + k], t[k]);
+      return (t[0] + t[1]) + (t[2] + t[3]);
+    };
+    for (int ik = rb; ik < di; ++ik) {
+      const int v0 = a.upd_ptr[ik], nu = a.upd_ptr[ik + 1] - v0;
+      double *Aik = rowblk + (size_t)(ik - rb) * BB;
+      const double *D = Dk + (size_t)(ik - rb) * BB;
+      for (int o = threadIdx.x; o < BB; o += blockDim.x) Lt[o] = dot(Aik + o % B, D + (o / B) * B);
+      __syncthreads();
+      for (int o = threadIdx.x; o < (nu + 1) * BB; o += blockDim.x) {
+        const int uu = o / BB - 1, r = o % BB;
+        if (uu < 0)
+          Aik[r] = Lt[r];
+        else
+          rowblk[(size_t)(a.upd[2 * (v0 + uu)] - rb) * BB + r] -=
+              dot(Lt + r % B, Ub + (size_t)(v0 - u0 + uu) * BB + (r / B) * B);
+      }
+      __syncthreads();
+    }
+    if (warp == 0) {
+      const double *Ad = rowblk + (size_t)(di - rb) * BB;
+      double w[B];
+#pragma unroll
+      for (int c = 0; c < B; ++c) w[c] = lane < B ? Ad[c * B + lane] : 0.;
+      bool un = lane < B, singular = false;
+      int pos = 0, mycol = 0;  // the step whose pivot row this lane is; the pivot row of step `lane`
+#pragma unroll
+      for (int k = 0; k < B; ++k) {
+        // largest magnitude (within 2^-15), first row on ties
+        const unsigned hi = (unsigned)__double2hiint(w[k]) & 0x7fffffffu;
+        const unsigned key = (un && hi < 0x7ff00000u) ? ((hi & ~31u) | (unsigned)(31 - lane)) : 0u;
+        const unsigned mb = __reduce_max_sync(0xffffffffu, key);
+        singular = singular || (mb >> 5) == 0u;
+        const int p = 31 - (int)(mb & 31u);
+        const bool me = lane == p;
+        const double ip = 1.0 / __shfl_sync(0xffffffffu, w[k], p), l = w[k];
+        mycol = lane == k ? p : mycol;
+        pos = me ? k : pos;
+        un = un && !me;
+#pragma unroll
+        for (int c = 0; c < B; ++c)
+          if (c != k) {
+            const double v = __shfl_sync(0xffffffffu, w[c], p) * ip;
+            w[c] = me ? v : fma(-l, v, w[c]);
+          }
+        w[k] = me ? ip : -l * ip;
+      }
+      if (singular && lane == 0) raise_err(a.err, DERR_SINGULAR_ILU);
+      double *Di = a.dinv + (size_t)i * BB;
+#pragma unroll
+      for (int c = 0; c < B; ++c) {
+        const int col = __shfl_sync(0xffffffffu, mycol, c);
+        if (lane < B) Di[col * B + pos] = w[c];
+      }
+    } else {
+      for (int o = threadIdx.x - 32; o < (re - rb) * BB; o += blockDim.x - 32) a.data[(size_t)rb * BB + o] = rowblk[o];
+    }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) publish_max(a.progress + g, a.tag | (unsigned long long)(slot + 1));
@@ -547,9 +857,34 @@ int sweep_occupancy_dispatch(int S, int block, size_t smem) {
     default: fail(EG_ERR_INVALID, "unsupported block size");
   }
 }
+// the block sizes of the compile-time kernels: every HDG degree, DG up to k = 2
+#define EG_ILU_SMALL(B, CALL)                                         \
+  switch (B) {                                                        \
+    case 4: { constexpr int BS = 4; CALL; } break;                    \
+    case 8: { constexpr int BS = 8; CALL; } break;                    \
+    case 12: { constexpr int BS = 12; CALL; } break;                  \
+    case 16: { constexpr int BS = 16; CALL; } break;                  \
+    case 20: { constexpr int BS = 20; CALL; } break;                  \
+    case 24: { constexpr int BS = 24; CALL; } break;                  \
+    case 28: { constexpr int BS = 28; CALL; } break;                  \
+    case 32: { constexpr int BS = 32; CALL; } break;                  \
+    case 36: { constexpr int BS = 36; CALL; } break;                  \
+    default: fail(EG_ERR_INVALID, "unsupported block size");          \
+  }
+bool factor_small(int B) { return B <= 32; }
+int small_sweep_occupancy(int B, int block, size_t smem) {
+  EG_ILU_SMALL(B, return std::min(per_sm(ilu_sweep_small_kernel<BS, false>, block, smem),
+                                  per_sm(ilu_sweep_small_kernel<BS, true>, block, smem)));
+  return 0;
+}
+int small_factor_occupancy(int B, size_t smem) {
+  EG_ILU_SMALL(B, if constexpr (BS <= 32) return per_sm(ilu_factor_small_kernel<BS>, 512, smem));
+  return 0;
+}
 int factor_occupancy(int B, bool staged, size_t smem) {
+  if (staged && factor_small(B)) return small_factor_occupancy(B, smem);
   if (staged)
-    return B <= 32 ? per_sm(ilu_factor_kernel<1, true>, 256, smem) : per_sm(ilu_factor_kernel<2, true>, 256, smem);
+    return per_sm(ilu_factor_kernel<2, true>, 256, smem);
   switch ((B + 31) / 32) {
     case 2: return per_sm(ilu_factor_kernel<2, false>, 256, 0);
     case 3: return per_sm(ilu_factor_kernel<3, false>, 256, 0);
@@ -655,8 +990,10 @@ void build_plan(Ctx &c, int form) {
   if (fill_src.empty()) fill_src.push_back(0);
   if (upd.empty()) upd.push_back(0);
   P.maxl = P.maxu = P.maxrow = 0;
+  P.maxtot = 1;
   for (int i = 0; i < P.rows; ++i) {
     P.maxl = std::max(P.maxl, diag[i] - row[i]);
+    P.maxtot = std::max(P.maxtot, upd_ptr[diag[i]] - upd_ptr[row[i]]);
     P.maxu = std::max(P.maxu, row[i + 1] - diag[i] - 1);
     P.maxrow = std::max(P.maxrow, row[i + 1] - row[i]);
   }
@@ -670,15 +1007,18 @@ void build_plan(Ctx &c, int form) {
   while ((size_t)(2 * P.ring) * P.B * sizeof(double) <= kRingBytes) P.ring *= 2;
   int W = 8;
   auto sweep_smem = [&](int w) {
-    return sizeof(double) * ((size_t)w * (P.staged ? kStageBlocks * BB : 0) + (size_t)w * 32 * S +
+    return sizeof(double) * ((size_t)w * (P.staged ? kStageBlocks * BB + kMaxDeps * P.B : 32 * S) +
                              (size_t)P.ring * P.B);
   };
   while (W > 1 && sweep_smem(W) > kSweepSmemBudget) --W;
   if (P.ring < 2 * W) fail(EG_ERR_INVALID, "block ILU ring too small");
   P.sweep_warps = W;
   P.sweep_smem = sweep_smem(W);
-  P.factor_smem = P.staged ? sizeof(double) * BB * (size_t)(P.maxrow + P.maxupd + 4) : 0;
-  const int occ = std::min(sweep_occupancy_dispatch(S, 32 * W, P.sweep_smem),
+  P.factor_smem = !P.staged ? 0
+                  : sizeof(double) * BB * (size_t)(factor_small(P.B) ? P.maxrow + P.maxl + P.maxtot + 1
+                                                                     : P.maxrow + P.maxupd + 4);
+  const int occ = std::min(P.staged ? small_sweep_occupancy(P.B, 32 * W, P.sweep_smem)
+                                    : sweep_occupancy_dispatch(S, 32 * W, P.sweep_smem),
                            factor_occupancy(P.B, P.staged != 0, P.factor_smem));
   if (occ < 1) fail(EG_ERR_INVALID, "block ILU kernels do not fit on an SM");
   const int G = std::min(P.chunks, std::min(occ, 2) * sms);
@@ -740,6 +1080,11 @@ void build_plan(Ctx &c, int form) {
   P.data = c.alloc_n<double>((size_t)P.nnzb * BB);
   P.dinv = c.alloc_n<double>((size_t)P.rows * BB);
   P.w = c.alloc_n<double>((size_t)P.rows * P.B);
+  if (P.staged) {
+    const size_t bytes = sizeof(uint4) * (size_t)P.rows * P.B;
+    P.slots = c.alloc(bytes);
+    EG_CUDA(cudaMemsetAsync(P.slots, 0, bytes, c.stream));
+  }
   // the condensation keeps all 16 panels per cell where the Schur action
   // streams them (same layout and arithmetic); otherwise the fill forms them
   if (hdg && c.geo.npan != 16) P.panels16 = c.alloc_n<double>((size_t)c.n * 16 * BB);
@@ -779,6 +1124,15 @@ void sweep(Ctx &c, IluPlan &P, const double *in, double *out) {
   a.staged = P.staged;
   a.limit_ns = P.wait_limit_ns;
   a.starve = P.starve;
+  a.slots = static_cast<uint4 *>(P.slots);
+  a.epoch = P.epoch;
+  if constexpr (S <= 2) {
+    if (P.staged) {
+      EG_ILU_SMALL(P.B, launch_coop(ilu_sweep_small_kernel<BS, BACK>, P.grid_sweep, 32 * P.sweep_warps, P.sweep_smem,
+                                    c.stream, a));
+      return;
+    }
+  }
   launch_coop(ilu_sweep_kernel<S, BACK>, P.grid_sweep, 32 * P.sweep_warps, P.sweep_smem, c.stream, a);
 }
 
@@ -822,13 +1176,19 @@ void factor_launch(Ctx &c, IluPlan &P) {
   a.tag = (unsigned long long)(++P.epoch) << 32;
   a.limit_ns = P.wait_limit_ns;
   a.starve = P.starve;
+  a.maxl = P.maxl;
+  a.maxtot = P.maxtot;
+  if (SMEM && factor_small(P.B)) {
+    EG_ILU_SMALL(P.B, if constexpr (BS <= 32)
+                          launch_coop(ilu_factor_small_kernel<BS>, P.grid_factor, 512, P.factor_smem, c.stream, a));
+    return;
+  }
   launch_coop(ilu_factor_kernel<RMAX, SMEM>, P.grid_factor, 256, SMEM ? P.factor_smem : 0, c.stream, a);
 }
 
 void factor_dispatch(Ctx &c, IluPlan &P) {
   if (P.staged) {
-    if (P.B <= 32) factor_launch<1, true>(c, P);
-    else factor_launch<2, true>(c, P);
+    factor_launch<2, true>(c, P);
     return;
   }
   switch ((P.B + 31) / 32) {
