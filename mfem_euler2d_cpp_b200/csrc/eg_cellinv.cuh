@@ -53,18 +53,21 @@ __device__ __forceinline__ double pivot_reciprocal(double x) {
 }
 
 // A shared-memory pair that the compiler may not keep in registers for the next
-// column of tiles: those registers hold the matrix.
+// column of tiles: those registers hold the matrix. The clobber keeps the load
+// behind the stores and barriers before it.
 __device__ __forceinline__ double2 lds_pair(const double *p) {
   double2 v;
   asm volatile("ld.volatile.shared.v2.f64 {%0, %1}, [%2];"
                : "=d"(v.x), "=d"(v.y)
-               : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))));
+               : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p)))
+               : "memory");
   return v;
 }
 
 __device__ __forceinline__ double lds_one(const double *p) {
   double v;
-  asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))));
+  asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p)))
+               : "memory");
   return v;
 }
 
