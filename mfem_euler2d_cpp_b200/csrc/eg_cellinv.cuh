@@ -66,24 +66,36 @@ __device__ __forceinline__ double2 lds_pair(const double *p) {
 
 __device__ __forceinline__ double lds_one(const double *p) {
   double v;
-  asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p)))
+  asm volatile("ld.volatile.shared.f64 %0, [%1];"
+               : "=d"(v)
+               : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p)))
                : "memory");
   return v;
 }
 
 constexpr double kMaxB = 64.;
 
-template <int Q, int WR_, int WC_>
+// Strides in doubles of a node's two Jacobians and of a face point's 4x4 matrix
+// in shared memory: 16-byte accesses by lanes over nodes and columns then use
+// all banks (at 32 and 16 every node started in the same one).
+constexpr int kJacStride = 34, kFaceStride = 18;
+
+template <int Q, int WR_, int WC_, int DED_ = 0>
 struct InvCfg {
   static constexpr int P = Q * Q, M = 4 * P, T = 4 * Q, MT = (M + 7) / 8;
-  static constexpr int WR = WR_, WC = WC_, THREADS = 32 * WR * WC;
+  // DED: one more warp, without tiles, inverts the pivot blocks (where the
+  // registers allow it); otherwise the tile warps take turns
+  static constexpr int WR = WR_, WC = WC_, DED = DED_, NW = WR * WC, THREADS = 32 * (NW + DED);
   static constexpr int TR = (MT + WR - 1) / WR, TC = (MT + WC - 1) / WC;  // tiles per warp
   // stride of the matrix in shared memory: LDA % 8 in {2, 6} makes a warp's
   // 8x8 tile accesses, and 16-byte accesses with lanes over columns, conflict-free
   static constexpr int LDA = (M % 8 == 0 || M % 8 == 4) ? M + 2 : M + 1;
   static_assert(LDA % 8 == 2 || LDA % 8 == 6, "tile accesses");
   static constexpr int PR = 8 * TR * WR, PC = 8 * TC * WC;  // rows and columns padded to whole warp grids
-  static constexpr int PANELS = 2 * (PR * 8 + 8 * PC);  // doubles of the double-buffered panel and pivot rows
+  // stride of the pivot rows: 64 bytes past a multiple of 128, so that the four
+  // rows an operand load touches use all banks
+  static constexpr int TS = PC % 16 == 0 ? PC + 8 : PC;
+  static constexpr int PANELS = 2 * (PR * 8 + 8 * TS);  // doubles of the double-buffered panel and pivot rows
   static constexpr int REGION = LDA * M > PANELS ? LDA * M : PANELS;
 };
 
@@ -147,23 +159,24 @@ struct Invert8 {
 // Sets *bad (shared) when the elimination cannot vouch for the result. Ends
 // with a CTA barrier.
 //
-// One barrier per panel. At its start one warp, another one each panel, forms
-// the next pivot block from the published tile (before this panel's update)
-// and inverts it; then it joins the update. The update has no branches: the
+// One barrier per panel. At its start one warp (C::DED, or another one each
+// panel) forms the next pivot block from the published tile (before this panel's update)
+// and inverts it; a tile warp then joins the update. The update has no branches: the
 // pivot column and row are set to zero first, the panel's pivot rows hold the
 // identity, and the right operand of the pivot column is the identity. Tiles
 // are updated in pairs, so that the two MMAs of a tile are not back to back
 // (26 cycles from one to the other, 16 between two of different tiles).
 template <class C>
 __device__ __forceinline__ void invert_tiles(double (&acc)[C::TR][C::TC][2], double *panels, double *tiles, int *bad) {
-  constexpr int MT = C::MT, PR = C::PR, PC = C::PC, WR = C::WR, WC = C::WC, TR = C::TR, TC = C::TC;
+  constexpr int MT = C::MT, PR = C::PR, TS = C::TS, WR = C::WR, WC = C::WC, TR = C::TR, TC = C::TC;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wr = warp % WR, wc = warp / WR;
   const int gq = lane >> 2, tq = lane & 3;
   double *Tis = tiles + 128;  // the inverse pivot blocks, double-buffered like the rest
+  const bool tiles_here = C::DED == 0 || warp < C::NW;
   bool fine = true;
-  // panel columns (negated), [row][8]; pivot rows, [8][PC]; the next diagonal tile, [8][8]
-  const auto pan = [&](int buf) { return panels + buf * (8 * PR + 8 * PC); };
-  const auto top = [&](int buf) { return panels + buf * (8 * PR + 8 * PC) + 8 * PR; };
+  // panel columns (negated), [row][8]; pivot rows, [8][TS]; the next diagonal tile, [8][8]
+  const auto pan = [&](int buf) { return panels + buf * (8 * PR + 8 * TS); };
+  const auto top = [&](int buf) { return panels + buf * (8 * PR + 8 * TS) + 8 * PR; };
   const auto publish = [&](int nxt, int buf) {
     if (nxt % WC == wc) {
 #pragma unroll
@@ -182,7 +195,7 @@ __device__ __forceinline__ void invert_tiles(double (&acc)[C::TR][C::TC][2], dou
 #pragma unroll
       for (int a = 0; a < TR; ++a)
         if (wr + a * WR == nxt) {
-          double *W = top(buf) + gq * PC + 2 * tq;
+          double *W = top(buf) + gq * TS + 2 * tq;
 #pragma unroll
           for (int b = 0; b < TC; ++b)
             *reinterpret_cast<double2 *>(W + (wc + b * WC) * 8) = make_double2(acc[a][b][0], acc[a][b][1]);
@@ -199,9 +212,11 @@ __device__ __forceinline__ void invert_tiles(double (&acc)[C::TR][C::TC][2], dou
         if ((WR != WC || a == b) && wr + a * WR == i && wc + b * WC == i)
           *reinterpret_cast<double2 *>(tiles + buf * 64 + gq * 8 + 2 * tq) = make_double2(acc[a][b][0], acc[a][b][1]);
   };
-  publish(0, 0);
-  publish_diagonal(0, 1);
-  publish_diagonal(1, 0);
+  if (tiles_here) {
+    publish(0, 0);
+    publish_diagonal(0, 1);
+    publish_diagonal(1, 0);
+  }
   __syncthreads();
   if (warp == 0) {
     Invert8 inv;
@@ -215,19 +230,19 @@ __device__ __forceinline__ void invert_tiles(double (&acc)[C::TR][C::TC][2], dou
   for (int p = 0; p < MT; ++p) {
     const int buf = p & 1;
     const double ti0 = Tis[buf * 64 + gq * 8 + tq], ti1 = Tis[buf * 64 + gq * 8 + tq + 4];
-    const double *P = pan(buf) + gq * 8 + 2 * tq, *W = top(buf) + tq * PC + gq;
+    const double *P = pan(buf) + gq * 8 + 2 * tq, *W = top(buf) + tq * TS + gq;
     // rows 2 tq and 2 tq + 1 of B = T^{-1} A_p,ct, column gq: the transposed
     // product, whose accumulator layout is the operand layout the update needs
     const auto pivot_rows = [&](int ct, double &b0, double &b1) {
       const bool pc = ct == p;
       const double t0 = pc ? (gq == tq ? 1. : 0.) : W[ct * 8];
-      const double t1 = pc ? (gq == tq + 4 ? 1. : 0.) : W[4 * PC + ct * 8];
+      const double t1 = pc ? (gq == tq + 4 ? 1. : 0.) : W[4 * TS + ct * 8];
       b0 = b1 = 0.;
       dmma_m8n8k4(b0, b1, t0, ti0);
       dmma_m8n8k4(b0, b1, t1, ti1);
       fine = fine && (pc || (fabs(b0) <= kMaxB && fabs(b1) <= kMaxB));
     };
-    if (warp == (p + 1) % (WR * WC) && p + 1 < MT) {
+    if (warp == (C::DED ? C::NW : (p + 1) % C::NW) && p + 1 < MT) {
       double b0, b1;
       pivot_rows(p + 1, b0, b1);
       const double2 w = *reinterpret_cast<const double2 *>(P + (p + 1) * 64);
@@ -240,54 +255,56 @@ __device__ __forceinline__ void invert_tiles(double (&acc)[C::TR][C::TC][2], dou
       inv.run(Tis + (buf ^ 1) * 64);
       fine = fine && inv.ok;
     }
-    if (p % WC == wc) {
+    if (tiles_here) {
+      if (p % WC == wc) {
 #pragma unroll
-      for (int b = 0; b < TC; ++b)
-        if (wc + b * WC == p) {
+        for (int b = 0; b < TC; ++b)
+          if (wc + b * WC == p) {
 #pragma unroll
-          for (int a = 0; a < TR; ++a) acc[a][b][0] = acc[a][b][1] = 0.;
-        }
-    }
-    if (p % WR == wr) {
-#pragma unroll
-      for (int a = 0; a < TR; ++a)
-        if (wr + a * WR == p) {
-#pragma unroll
-          for (int b = 0; b < TC; ++b) acc[a][b][0] = acc[a][b][1] = 0.;
-        }
-    }
-    double b0, b1;
-    pivot_rows(wc, b0, b1);
-#pragma unroll
-    for (int b = 0; b < TC; ++b) {
-      // the next column's rows of B are formed between this column's updates
-      const int cn = wc + (b + 1 < TC ? b + 1 : b) * WC;
-      const bool pc = cn == p;
-      double t0 = lds_one(W + cn * 8), t1 = lds_one(W + 4 * PC + cn * 8), n0 = 0., n1 = 0.;
-#pragma unroll
-      for (int a = 0; a < TR; a += 2) {
-        const double2 w = lds_pair(P + (wr + a * WR) * 64);
-        if (a + 1 < TR) {
-          const double2 x = lds_pair(P + (wr + (a + 1) * WR) * 64);
-          dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.x, b0);
-          dmma_m8n8k4(acc[a + 1][b][0], acc[a + 1][b][1], x.x, b0);
-          dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.y, b1);
-          dmma_m8n8k4(acc[a + 1][b][0], acc[a + 1][b][1], x.y, b1);
-        } else {
-          dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.x, b0);
-          dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.y, b1);
-        }
-        if (b + 1 < TC && a == 0) dmma_m8n8k4(n0, n1, pc ? (gq == tq ? 1. : 0.) : t0, ti0);
-        if (b + 1 < TC && (a == 2 || TR <= 2)) dmma_m8n8k4(n0, n1, pc ? (gq == tq + 4 ? 1. : 0.) : t1, ti1);
+            for (int a = 0; a < TR; ++a) acc[a][b][0] = acc[a][b][1] = 0.;
+          }
       }
-      if (b + 1 < TC) {
-        fine = fine && (pc || (fabs(n0) <= kMaxB && fabs(n1) <= kMaxB));
-        b0 = n0;
-        b1 = n1;
+      if (p % WR == wr) {
+#pragma unroll
+        for (int a = 0; a < TR; ++a)
+          if (wr + a * WR == p) {
+#pragma unroll
+            for (int b = 0; b < TC; ++b) acc[a][b][0] = acc[a][b][1] = 0.;
+          }
       }
+      double b0, b1;
+      pivot_rows(wc, b0, b1);
+#pragma unroll
+      for (int b = 0; b < TC; ++b) {
+        // the next column's rows of B are formed between this column's updates
+        const int cn = wc + (b + 1 < TC ? b + 1 : b) * WC;
+        const bool pc = cn == p;
+        double t0 = lds_one(W + cn * 8), t1 = lds_one(W + 4 * TS + cn * 8), n0 = 0., n1 = 0.;
+#pragma unroll
+        for (int a = 0; a < TR; a += 2) {
+          const double2 w = lds_pair(P + (wr + a * WR) * 64);
+          if (a + 1 < TR) {
+            const double2 x = lds_pair(P + (wr + (a + 1) * WR) * 64);
+            dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.x, b0);
+            dmma_m8n8k4(acc[a + 1][b][0], acc[a + 1][b][1], x.x, b0);
+            dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.y, b1);
+            dmma_m8n8k4(acc[a + 1][b][0], acc[a + 1][b][1], x.y, b1);
+          } else {
+            dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.x, b0);
+            dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.y, b1);
+          }
+          if (b + 1 < TC && a == 0) dmma_m8n8k4(n0, n1, pc ? (gq == tq ? 1. : 0.) : t0, ti0);
+          if (b + 1 < TC && (a == 2 || TR <= 2)) dmma_m8n8k4(n0, n1, pc ? (gq == tq + 4 ? 1. : 0.) : t1, ti1);
+        }
+        if (b + 1 < TC) {
+          fine = fine && (pc || (fabs(n0) <= kMaxB && fabs(n1) <= kMaxB));
+          b0 = n0;
+          b1 = n1;
+        }
+      }
+      publish(p + 1, buf ^ 1);
+      publish_diagonal(p + 2, buf ^ 1);
     }
-    publish(p + 1, buf ^ 1);
-    publish_diagonal(p + 2, buf ^ 1);
     __syncthreads();
   }
   if (!fine) *bad = 1;
@@ -315,6 +332,7 @@ template <class C>
 __device__ __forceinline__ void store_tiles(const double (&acc)[C::TR][C::TC][2], double *A) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wr = warp % C::WR, wc = warp / C::WR;
   const int gq = lane >> 2, tq = lane & 3;
+  if (C::DED && warp >= C::NW) return;
 #pragma unroll
   for (int a = 0; a < C::TR; ++a)
 #pragma unroll
@@ -352,8 +370,8 @@ __device__ __forceinline__ void jacobian_axis(const double *u, int axis, double 
   j[15] = vn * gm1 + vn;
 }
 
-// Flux Jacobians of the cell's nodes, J[node][axis][16] (column-major 4x4),
-// scaled by -dt w of the node.
+// Flux Jacobians of the cell's nodes, J[node * kJacStride + 16 axis + k]
+// (column-major 4x4), scaled by -dt w of the node.
 template <int Q>
 __device__ __forceinline__ void node_jacobians(double *J, const STab<Q> &st, const double *us, const Geo &g) {
   for (int t = threadIdx.x; t < 2 * Q * Q; t += blockDim.x) {
@@ -362,58 +380,53 @@ __device__ __forceinline__ void node_jacobians(double *J, const STab<Q> &st, con
     jacobian_axis(us + 4 * node, axis, g.gm1, j);
     const double s = -g.dt * st.w(node);
 #pragma unroll
-    for (int k = 0; k < 16; ++k) J[t * 16 + k] = s * j[k];
+    for (int k = 0; k < 16; ++k) J[node * kJacStride + 16 * axis + k] = s * j[k];
   }
 }
 
-// The cell matrix of build_cell_matrix (eg_cellmat.cuh), one 4x4 node block
-// per thread: node jn meets the nodes on its x-line and y-line only, 2 q - 1 of
-// q^2; the other blocks are zero. J from node_jacobians. Starts with a CTA
-// barrier between the zeros and the blocks and needs one before use.
+// The cell matrix of build_cell_matrix (eg_cellmat.cuh), one column of a 4x4
+// node block per thread: node jn meets the nodes on its x-line and y-line only,
+// 2 q - 1 of q^2; the other blocks are zero. Lanes run over the columns, which
+// keeps the stores free of bank conflicts (a whole block per thread: 16-way).
+// J from node_jacobians. Starts with a CTA barrier between the zeros and the
+// blocks and needs one before use.
 template <class C, int Q>
 __device__ __forceinline__ void assemble_cell(double *A, const STab<Q> &st, const double *J, const double *FM,
                                               const Geo &g) {
-  constexpr int M = C::M, LDA = C::LDA, L = 2 * Q - 1, P = Q * Q;
+  constexpr int M = C::M, LDA = C::LDA, L = 2 * Q - 1;
   double2 *A2 = reinterpret_cast<double2 *>(A);
   for (int i = threadIdx.x; i < LDA * M / 2; i += blockDim.x) A2[i] = make_double2(0., 0.);
   __syncthreads();
   const double sx = g.dt * g.hy / g.area, sy = g.dt * g.hx / g.area;
-  for (int t = threadIdx.x; t < P * L; t += blockDim.x) {
+  for (int t = threadIdx.x; t < M * L; t += blockDim.x) {
     // pos < Q: x-line node pos; else the y-line node pos - Q, past the own one
-    const int jn = t % P, pos = t / P, jx = jn % Q, jy = jn / Q;
+    const int col = t % M, pos = t / M, jn = col >> 2, d = col & 3, jx = jn % Q, jy = jn / Q;
     const bool xl = pos < Q, own = xl && pos == jx;
     const int iy0 = pos - Q, ix = xl ? pos : jx, iy = xl ? jy : iy0 + (iy0 >= jy ? 1 : 0);
     const int i = iy * Q + ix;
     const double im = st.inv_mass(i);
-    double v[16];
-    const auto line = [&](bool first, double gd, double w0, double w1, const double *j, const double *m0,
-                          const double *m1) {
+    double v[4] = {own && d == 0 ? 1. : 0., own && d == 1 ? 1. : 0., own && d == 2 ? 1. : 0., own && d == 3 ? 1. : 0.};
+    const auto line = [&](double gd, double w0, double w1, const double *j, const double *m0, const double *m1) {
 #pragma unroll
-      for (int k = 0; k < 16; k += 2) {
+      for (int k = 0; k < 4; k += 2) {
         const double2 a = *reinterpret_cast<const double2 *>(j + k), b = *reinterpret_cast<const double2 *>(m0 + k),
                       c = *reinterpret_cast<const double2 *>(m1 + k);
-        v[k] = (first ? 0. : v[k]) + (gd * a.x + (w0 * b.x + w1 * c.x));
-        v[k + 1] = (first ? 0. : v[k + 1]) + (gd * a.y + (w0 * b.y + w1 * c.y));
+        v[k] += gd * a.x + (w0 * b.x + w1 * c.x);
+        v[k + 1] += gd * a.y + (w0 * b.y + w1 * c.y);
       }
     };
+    const double *j = J + kJacStride * jn + 4 * d, *m = FM + 4 * d;
     if (xl) {
       const double e = im * sx * st.ew(jy), f0 = st.fb(0, jy, ix) * st.fb(0, jy, jx), f1 = st.fb(1, jy, ix) * st.fb(1, jy, jx);
-      line(true, im * st.tdx(jx, ix), e * f0, e * f1, J + 32 * jn, FM + jy * 16, FM + (Q + jy) * 16);
+      line(im * st.tdx(jx, ix), e * f0, e * f1, j, m + kFaceStride * jy, m + kFaceStride * (Q + jy));
     }
     if (!xl || own) {
       const double e = im * sy * st.ew(jx), f2 = st.fb(2, jx, iy) * st.fb(2, jx, jy), f3 = st.fb(3, jx, iy) * st.fb(3, jx, jy);
-      line(!xl, im * st.tdy(jy, iy), e * f2, e * f3, J + 32 * jn + 16, FM + (2 * Q + jx) * 16, FM + (3 * Q + jx) * 16);
+      line(im * st.tdy(jy, iy), e * f2, e * f3, j + 16, m + kFaceStride * (2 * Q + jx), m + kFaceStride * (3 * Q + jx));
     }
-    if (own) {
-#pragma unroll
-      for (int k = 0; k < 16; k += 5) v[k] += 1.;
-    }
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-      double2 *a = reinterpret_cast<double2 *>(A + (size_t)(4 * jn + d) * LDA + 4 * i);
-      a[0] = make_double2(v[4 * d], v[4 * d + 1]);
-      a[1] = make_double2(v[4 * d + 2], v[4 * d + 3]);
-    }
+    double2 *a = reinterpret_cast<double2 *>(A + (size_t)col * LDA + 4 * i);
+    a[0] = make_double2(v[0], v[1]);
+    a[1] = make_double2(v[2], v[3]);
   }
 }
 

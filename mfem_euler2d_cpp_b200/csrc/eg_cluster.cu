@@ -23,14 +23,16 @@ namespace cg = cooperative_groups;
 namespace eg {
 namespace {
 
-template <int Q, int WR_, int WC_, int CL_>
+template <int Q, int WR_, int WC_, int CL_, int DED_>
 struct ClCfg {
   static constexpr int P = Q * Q, M = 4 * P, T = 4 * Q, MT = (M + 7) / 8, CL = CL_;
-  static constexpr int WR = WR_, WC = WC_, THREADS = 32 * WR * WC;
+  // DED as in InvCfg
+  static constexpr int WR = WR_, WC = WC_, DED = DED_, NW = WR * WC, THREADS = 32 * (NW + DED);
   static constexpr int CT = (MT + CL - 1) / CL;                           // column tiles per CTA
   static constexpr int TR = (MT + WR - 1) / WR, TC = (CT + WC - 1) / WC;  // tiles per warp
   static constexpr int PR = 8 * TR * WR, PC = 8 * TC * WC;
-  static constexpr int PANELS = 2 * (8 * PR + 8 * PC);
+  static constexpr int TS = PC % 16 == 0 ? PC + 8 : PC;  // as in InvCfg
+  static constexpr int PANELS = 2 * (8 * PR + 8 * TS);
 };
 
 // acc: the CTA's tiles (rows wr + a WR, global columns rank + CL (wc + b WC))
@@ -41,14 +43,15 @@ struct ClCfg {
 template <class C>
 __device__ __forceinline__ void invert_tiles_cluster(double (&acc)[C::TR][C::TC][2], double *panels, double *tiles,
                                                      int *bad, cg::cluster_group &cluster) {
-  constexpr int MT = C::MT, PR = C::PR, PC = C::PC, WR = C::WR, WC = C::WC, TR = C::TR, TC = C::TC, CL = C::CL;
+  constexpr int MT = C::MT, PR = C::PR, TS = C::TS, WR = C::WR, WC = C::WC, TR = C::TR, TC = C::TC, CL = C::CL;
   const int rank = (int)cluster.block_rank();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wr = warp % WR, wc = warp / WR;
   const int gq = lane >> 2, tq = lane & 3;
   double *Tis = tiles + 128;
+  const bool tiles_here = C::DED == 0 || warp < C::NW;
   bool fine = true;
-  const auto pan = [&](int buf) { return panels + buf * (8 * PR + 8 * PC); };
-  const auto top = [&](int buf) { return panels + buf * (8 * PR + 8 * PC) + 8 * PR; };
+  const auto pan = [&](int buf) { return panels + buf * (8 * PR + 8 * TS); };
+  const auto top = [&](int buf) { return panels + buf * (8 * PR + 8 * TS) + 8 * PR; };
   const auto publish = [&](int nxt, int buf) {
     const int lt = nxt / CL;
     if (nxt % CL == rank && lt % WC == wc) {
@@ -73,7 +76,7 @@ __device__ __forceinline__ void invert_tiles_cluster(double (&acc)[C::TR][C::TC]
 #pragma unroll
       for (int a = 0; a < TR; ++a)
         if (wr + a * WR == nxt) {
-          double *W = top(buf) + gq * PC + 2 * tq;
+          double *W = top(buf) + gq * TS + 2 * tq;
 #pragma unroll
           for (int b = 0; b < TC; ++b)
             *reinterpret_cast<double2 *>(W + (wc + b * WC) * 8) = make_double2(acc[a][b][0], acc[a][b][1]);
@@ -100,9 +103,11 @@ __device__ __forceinline__ void invert_tiles_cluster(double (&acc)[C::TR][C::TC]
     for (int r = 0; r < CL; ++r)
       if (r != rank) *reinterpret_cast<double2 *>(cluster.map_shared_rank(Ti + 2 * lane, r)) = v;
   };
-  publish(0, 0);
-  publish_diagonal(0, 1);
-  publish_diagonal(1, 0);
+  if (tiles_here) {
+    publish(0, 0);
+    publish_diagonal(0, 1);
+    publish_diagonal(1, 0);
+  }
   cluster.sync();
   if (rank == 0 && warp == 0) {
     Invert8 inv;
@@ -117,17 +122,17 @@ __device__ __forceinline__ void invert_tiles_cluster(double (&acc)[C::TR][C::TC]
   for (int p = 0; p < MT; ++p) {
     const int buf = p & 1;
     const double ti0 = Tis[buf * 64 + gq * 8 + tq], ti1 = Tis[buf * 64 + gq * 8 + tq + 4];
-    const double *P = pan(buf) + gq * 8 + 2 * tq, *W = top(buf) + tq * PC + gq;
+    const double *P = pan(buf) + gq * 8 + 2 * tq, *W = top(buf) + tq * TS + gq;
     const auto pivot_rows = [&](int lt, double &b0, double &b1) {
       const bool pc = rank + CL * lt == p;
       const double t0 = pc ? (gq == tq ? 1. : 0.) : lds_one(W + lt * 8);
-      const double t1 = pc ? (gq == tq + 4 ? 1. : 0.) : lds_one(W + 4 * PC + lt * 8);
+      const double t1 = pc ? (gq == tq + 4 ? 1. : 0.) : lds_one(W + 4 * TS + lt * 8);
       b0 = b1 = 0.;
       dmma_m8n8k4(b0, b1, t0, ti0);
       dmma_m8n8k4(b0, b1, t1, ti1);
       fine = fine && (pc || (fabs(b0) <= kMaxB && fabs(b1) <= kMaxB));
     };
-    if (p + 1 < MT && (p + 1) % CL == rank && warp == ((p + 1) / CL) % (WR * WC)) {
+    if (p + 1 < MT && (p + 1) % CL == rank && warp == (C::DED ? C::NW : ((p + 1) / CL) % C::NW)) {
       double b0, b1;
       pivot_rows((p + 1) / CL, b0, b1);
       const double2 w = *reinterpret_cast<const double2 *>(P + (p + 1) * 64);
@@ -141,47 +146,49 @@ __device__ __forceinline__ void invert_tiles_cluster(double (&acc)[C::TR][C::TC]
       send_inverse(Tis + (buf ^ 1) * 64);
       fine = fine && inv.ok;
     }
-    if (p % CL == rank && (p / CL) % WC == wc) {
+    if (tiles_here) {
+      if (p % CL == rank && (p / CL) % WC == wc) {
 #pragma unroll
-      for (int b = 0; b < TC; ++b)
-        if (wc + b * WC == p / CL) {
+        for (int b = 0; b < TC; ++b)
+          if (wc + b * WC == p / CL) {
 #pragma unroll
-          for (int a = 0; a < TR; ++a) acc[a][b][0] = acc[a][b][1] = 0.;
-        }
-    }
-    if (p % WR == wr) {
-#pragma unroll
-      for (int a = 0; a < TR; ++a)
-        if (wr + a * WR == p) {
-#pragma unroll
-          for (int b = 0; b < TC; ++b) acc[a][b][0] = acc[a][b][1] = 0.;
-        }
-    }
-    double b0, b1;
-    pivot_rows(wc, b0, b1);
-#pragma unroll
-    for (int b = 0; b < TC; ++b) {
-      double n0 = 0., n1 = 0.;
-#pragma unroll
-      for (int a = 0; a < TR; a += 2) {
-        const double2 w = lds_pair(P + (wr + a * WR) * 64);
-        if (a + 1 < TR) {
-          const double2 x = lds_pair(P + (wr + (a + 1) * WR) * 64);
-          dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.x, b0);
-          dmma_m8n8k4(acc[a + 1][b][0], acc[a + 1][b][1], x.x, b0);
-          dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.y, b1);
-          dmma_m8n8k4(acc[a + 1][b][0], acc[a + 1][b][1], x.y, b1);
-        } else {
-          dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.x, b0);
-          dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.y, b1);
-        }
-        if (b + 1 < TC && a == 0) pivot_rows(wc + (b + 1) * WC, n0, n1);
+            for (int a = 0; a < TR; ++a) acc[a][b][0] = acc[a][b][1] = 0.;
+          }
       }
-      b0 = n0;
-      b1 = n1;
+      if (p % WR == wr) {
+#pragma unroll
+        for (int a = 0; a < TR; ++a)
+          if (wr + a * WR == p) {
+#pragma unroll
+            for (int b = 0; b < TC; ++b) acc[a][b][0] = acc[a][b][1] = 0.;
+          }
+      }
+      double b0, b1;
+      pivot_rows(wc, b0, b1);
+#pragma unroll
+      for (int b = 0; b < TC; ++b) {
+        double n0 = 0., n1 = 0.;
+#pragma unroll
+        for (int a = 0; a < TR; a += 2) {
+          const double2 w = lds_pair(P + (wr + a * WR) * 64);
+          if (a + 1 < TR) {
+            const double2 x = lds_pair(P + (wr + (a + 1) * WR) * 64);
+            dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.x, b0);
+            dmma_m8n8k4(acc[a + 1][b][0], acc[a + 1][b][1], x.x, b0);
+            dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.y, b1);
+            dmma_m8n8k4(acc[a + 1][b][0], acc[a + 1][b][1], x.y, b1);
+          } else {
+            dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.x, b0);
+            dmma_m8n8k4(acc[a][b][0], acc[a][b][1], w.y, b1);
+          }
+          if (b + 1 < TC && a == 0) pivot_rows(wc + (b + 1) * WC, n0, n1);
+        }
+        b0 = n0;
+        b1 = n1;
+      }
+      publish(p + 1, buf ^ 1);
+      publish_diagonal(p + 2, buf ^ 1);
     }
-    publish(p + 1, buf ^ 1);
-    publish_diagonal(p + 2, buf ^ 1);
     cluster.sync();
   }
   if (!fine)
@@ -210,15 +217,16 @@ __device__ __forceinline__ void assemble_tiles(double (&acc)[C::TR][C::TC][2], c
         if (iy == jy) {
           const double e = im * sx * st.ew(jy), gd = im * st.tdx(jx, ix);
           const double f0 = e * (st.fb(0, jy, ix) * st.fb(0, jy, jx)), f1 = e * (st.fb(1, jy, ix) * st.fb(1, jy, jx));
-          const double *j = J + 32 * jn + 4 * d + c, *m0 = FM + jy * 16 + 4 * d + c, *m1 = FM + (Q + jy) * 16 + 4 * d + c;
+          const double *j = J + kJacStride * jn + 4 * d + c, *m0 = FM + jy * kFaceStride + 4 * d + c,
+                       *m1 = FM + (Q + jy) * kFaceStride + 4 * d + c;
           v0 += gd * j[0] + (f0 * m0[0] + f1 * m1[0]);
           v1 += gd * j[4] + (f0 * m0[4] + f1 * m1[4]);
         }
         if (ix == jx) {
           const double e = im * sy * st.ew(jx), gd = im * st.tdy(jy, iy);
           const double f2 = e * (st.fb(2, jx, iy) * st.fb(2, jx, jy)), f3 = e * (st.fb(3, jx, iy) * st.fb(3, jx, jy));
-          const double *j = J + 32 * jn + 16 + 4 * d + c, *m2 = FM + (2 * Q + jx) * 16 + 4 * d + c,
-                       *m3 = FM + (3 * Q + jx) * 16 + 4 * d + c;
+          const double *j = J + kJacStride * jn + 16 + 4 * d + c, *m2 = FM + (2 * Q + jx) * kFaceStride + 4 * d + c,
+                       *m3 = FM + (3 * Q + jx) * kFaceStride + 4 * d + c;
           v0 += gd * j[0] + (f2 * m2[0] + f3 * m3[0]);
           v1 += gd * j[4] + (f2 * m2[4] + f3 * m3[4]);
         }
@@ -234,6 +242,7 @@ template <class C>
 __device__ __forceinline__ void write_tiles(const double (&acc)[C::TR][C::TC][2], double *S, int rank) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wr = warp % C::WR, wc = warp / C::WR;
   const int gq = lane >> 2, tq = lane & 3;
+  if (C::DED && warp >= C::NW) return;
 #pragma unroll
   for (int a = 0; a < C::TR; ++a)
 #pragma unroll
@@ -270,13 +279,13 @@ __device__ __forceinline__ void lift_row_global(const double *lift, const double
 // cluster's scratch (L2-resident: 22 to 28 MB over all clusters) and the CTAs
 // share the outputs: the columns of X, the rows of y, the four sides' C_s R_s
 // A^{-1} and panels.
-template <int Q, int WR, int WC, int CL>
-__global__ void __launch_bounds__(32 * WR *WC, 1)
+template <int Q, int WR, int WC, int CL, int DED>
+__global__ void __launch_bounds__(32 * (WR * WC + DED), 1)
     condense_cluster_kernel(Geo g, const double *__restrict__ tab, Frozen fz, const double *__restrict__ u,
                             const double *__restrict__ r, double *XY, double *Cb, double *sf_out, double *contrib,
                             double *panels, double *scratch, int *redo, int *redo_count) {
-  using C = ClCfg<Q, WR, WC, CL>;
-  constexpr int M = C::M, T = C::T, NR = 4 * T + 1;
+  using C = ClCfg<Q, WR, WC, CL, DED>;
+  constexpr int M = C::M, T = C::T, NR = 4 * T + 1, TS = T + 2;
   __shared__ CondenseInvShared<Q> sh;
   __shared__ __align__(16) double tiles[256];
   extern __shared__ __align__(16) double dyn[];
@@ -349,11 +358,11 @@ __global__ void __launch_bounds__(32 * WR *WC, 1)
           v[2] += f * p1[l].x;
           v[3] += f * p1[l].y;
         }
-        const double *cb = sh.CB + (s * Q + jj) * 16;
+        const double *cb = sh.CB + (s * Q + jj) * kFaceStride;
         double o[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) o[c] = (cb[c] * v[0] + cb[c + 4] * v[1]) + (cb[c + 8] * v[2] + cb[c + 12] * v[3]);
-        double2 *dst = reinterpret_cast<double2 *>(aux + (size_t)col * T + 4 * jj);
+        double2 *dst = reinterpret_cast<double2 *>(aux + (size_t)col * TS + 4 * jj);
         dst[0] = make_double2(o[0], o[1]);
         dst[1] = make_double2(o[2], o[3]);
       }
@@ -361,7 +370,7 @@ __global__ void __launch_bounds__(32 * WR *WC, 1)
       for (int t = threadIdx.x; t < T * T; t += blockDim.x) {
         const int row = t % T, jc = t / T;
         double x[4];
-        lift_row<Q>(sh.lift, aux + row, T, jc, x);
+        lift_row<Q>(sh.lift, aux + row, TS, jc, x);
 #pragma unroll
         for (int o = 0; o < 4; ++o) panels[(((size_t)e * 16 + s * 4 + o) * T + jc) * T + row] = x[o];
       }
@@ -376,7 +385,7 @@ __global__ void __launch_bounds__(32 * WR *WC, 1)
 #pragma unroll
           for (int d = 0; d < 4; ++d) v[d] += f * p[d];
         }
-        const double *cb = sh.CB + t * 16;
+        const double *cb = sh.CB + t * kFaceStride;
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           contrib[(size_t)e * 4 * T + 4 * t + c] = (cb[c] * v[0] + cb[c + 4] * v[1]) + (cb[c + 8] * v[2] + cb[c + 12] * v[3]);
@@ -386,14 +395,14 @@ __global__ void __launch_bounds__(32 * WR *WC, 1)
 }
 
 // Explicit DG block-Jacobi inverses, column-major.
-template <int Q, int WR, int WC, int CL>
-__global__ void __launch_bounds__(32 * WR *WC, 1)
+template <int Q, int WR, int WC, int CL, int DED>
+__global__ void __launch_bounds__(32 * (WR * WC + DED), 1)
     dg_inverse_cluster_kernel(Geo g, const double *__restrict__ tab, Frozen fz, const double *__restrict__ u,
                               double *inv, int *redo, int *redo_count) {
-  using C = ClCfg<Q, WR, WC, CL>;
+  using C = ClCfg<Q, WR, WC, CL, DED>;
   constexpr int M = C::M;
   __shared__ STab<Q> st;
-  __shared__ __align__(16) double us[M], UT[16 * Q], FM[64 * Q], tiles[256];
+  __shared__ __align__(16) double us[M], UT[16 * Q], FM[4 * Q * kFaceStride], tiles[256];
   __shared__ int bad;
   extern __shared__ __align__(16) double dyn[];
   double *J = dyn + C::PANELS;
@@ -408,7 +417,7 @@ __global__ void __launch_bounds__(32 * WR *WC, 1)
     cell_traces<Q>(st, us, UT);
     node_jacobians<Q>(J, st, us, g);
     __syncthreads();
-    dg_face_matrices<Q>(UT, FM, g, fz, e);
+    dg_face_matrices<Q, kFaceStride>(UT, FM, g, fz, e);
     __syncthreads();
     double acc[C::TR][C::TC][2];
     assemble_tiles<C, Q>(acc, st, J, FM, g, rank);
@@ -458,12 +467,12 @@ int resident_clusters(Kern kern, int CL, int threads, size_t dyn) {
   return n;
 }
 
-template <int Q, int WR, int WC, int CL>
+template <int Q, int WR, int WC, int CL, int DED>
 void condense_launch(Ctx &c, const double *u, const double *r) {
-  using C = ClCfg<Q, WR, WC, CL>;
-  constexpr int AUX = 32 * C::P > C::M * C::T ? 32 * C::P : C::M * C::T;
+  using C = ClCfg<Q, WR, WC, CL, DED>;
+  constexpr int AUX = kJacStride * C::P > C::M * (C::T + 2) ? kJacStride * C::P : C::M * (C::T + 2);
   constexpr size_t dyn = sizeof(double) * (size_t)(C::PANELS + AUX);
-  auto kern = condense_cluster_kernel<Q, WR, WC, CL>;
+  auto kern = condense_cluster_kernel<Q, WR, WC, CL, DED>;
   const int clusters = std::min(c.n, resident_clusters(kern, CL, C::THREADS, dyn));
   if (c.work_gj == nullptr || c.work_gj_slots < clusters) {
     c.work_gj = c.alloc_n<double>((size_t)clusters * C::M * C::M);
@@ -473,11 +482,11 @@ void condense_launch(Ctx &c, const double *u, const double *r) {
                  Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, r, c.XY, c.Cb, c.sf, c.contrib, c.panels, c.work_gj,
                  c.redo, c.derr + 3);
 }
-template <int Q, int WR, int WC, int CL>
+template <int Q, int WR, int WC, int CL, int DED>
 void dg_launch(Ctx &c, const double *u) {
-  using C = ClCfg<Q, WR, WC, CL>;
-  constexpr size_t dyn = sizeof(double) * (size_t)(C::PANELS + 32 * C::P);
-  auto kern = dg_inverse_cluster_kernel<Q, WR, WC, CL>;
+  using C = ClCfg<Q, WR, WC, CL, DED>;
+  constexpr size_t dyn = sizeof(double) * (size_t)(C::PANELS + kJacStride * C::P);
+  auto kern = dg_inverse_cluster_kernel<Q, WR, WC, CL, DED>;
   const int clusters = std::min(c.n, resident_clusters(kern, CL, C::THREADS, dyn));
   launch_cluster(kern, CL, C::THREADS, dyn, clusters, c.stream, c.geo, (const double *)c.tab,
                  Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, c.pc_dg, c.redo, c.derr + 3);
@@ -486,21 +495,24 @@ void dg_launch(Ctx &c, const double *u) {
 }  // namespace
 
 // Shapes: the fewest CTAs whose registers hold the matrix without spills (k = 6:
-// 49 tiles for each of 8 warps; k = 7: 16 for 16; k = 8: 28 for 12). Clusters
-// of 2 fill all 148 SMs, of 4 and 6 132.
+// 35 tiles for each of 10 warps and one more for the pivot blocks; k = 7: 16
+// for 16; k = 8: 28 for 12). Clusters of 2 fill all 148 SMs, of 4 and 6 132.
+// Condensation with a warp for the pivot blocks against tile warps in turn:
+// 8.10 against 9.12 ms at k = 6 (64x64 cells), but 5.21 against 4.74 at k = 7
+// and 13.3 against 11.8 at k = 8 (32x32), where it costs the others registers.
 void launch_condense_cluster(Ctx &c, const double *u, const double *r) {
   switch (c.q) {
-    case 7: condense_launch<7, 4, 2, 2>(c, u, r); break;
-    case 8: condense_launch<8, 4, 4, 4>(c, u, r); break;
-    case 9: condense_launch<9, 6, 2, 6>(c, u, r); break;
+    case 7: condense_launch<7, 5, 2, 2, 1>(c, u, r); break;
+    case 8: condense_launch<8, 4, 4, 4, 0>(c, u, r); break;
+    case 9: condense_launch<9, 6, 2, 6, 0>(c, u, r); break;
     default: fail(EG_ERR_INVALID, "unsupported degree");
   }
 }
 void launch_dg_inverse_cluster(Ctx &c, const double *u) {
   switch (c.q) {
-    case 7: dg_launch<7, 4, 2, 2>(c, u); break;
-    case 8: dg_launch<8, 4, 4, 4>(c, u); break;
-    case 9: dg_launch<9, 6, 2, 6>(c, u); break;
+    case 7: dg_launch<7, 5, 2, 2, 1>(c, u); break;
+    case 8: dg_launch<8, 4, 4, 4, 0>(c, u); break;
+    case 9: dg_launch<9, 6, 2, 6, 0>(c, u); break;
     default: fail(EG_ERR_INVALID, "unsupported degree");
   }
 }

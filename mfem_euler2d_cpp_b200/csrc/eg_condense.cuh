@@ -10,7 +10,7 @@ template <int Q>
 struct CondenseInvShared {
   static constexpr int M = 4 * Q * Q;
   STab<Q> st;
-  alignas(16) double us[M], rs[M], y[M], UT[16 * Q], FM[64 * Q], CB[64 * Q], SF[4 * Q], lift[4 * Q * Q];
+  alignas(16) double us[M], rs[M], y[M], UT[16 * Q], FM[4 * Q * kFaceStride], CB[4 * Q * kFaceStride], SF[4 * Q], lift[4 * Q * Q];
   int bad;
 };
 
@@ -42,8 +42,8 @@ __device__ __forceinline__ void condense_cell_data(CondenseInvShared<Q> &sh, con
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
       const double v = nsign * jm[k] + ((k % 5) == 0 ? stab : 0.);
-      sh.FM[task * 16 + k] = v;
-      sh.CB[task * 16 + k] = -ewj * v;
+      sh.FM[task * kFaceStride + k] = v;
+      sh.CB[task * kFaceStride + k] = -ewj * v;
     }
     const double sv = -(g.dt * (s < 2 ? g.hy : g.hx) / g.area * ewj) * stab;
     sh.SF[task] = sv;
@@ -55,7 +55,7 @@ __device__ __forceinline__ void condense_cell_data(CondenseInvShared<Q> &sh, con
   }
   __syncthreads();
   if (store)
-    for (int i = threadIdx.x; i < 64 * Q; i += blockDim.x) Cb[(size_t)e * 64 * Q + i] = sh.CB[i];
+    for (int i = threadIdx.x; i < 64 * Q; i += blockDim.x) Cb[(size_t)e * 64 * Q + i] = sh.CB[i / 16 * kFaceStride + i % 16];
 }
 
 // Row r of V B for the four sides, from a matrix V whose column c starts at V

@@ -207,19 +207,28 @@ __global__ void __launch_bounds__(256)
 // than eliminating the 4t + 1 right-hand sides (2 m^3 against m^3 + 2 m^2
 // (4t + 1): 2.0 against 2.6 M at k = 4), needs no registers for them, and the
 // matrix fits an SM twice at k = 4.
+// Bound by the FP64 tensor pipe while a cell is inverted and by shared memory
+// while it is assembled and its panels are formed; several cells per SM overlap
+// the two. Whole condensation, against the elimination of the right-hand sides
+// this replaces, ms: k = 1 0.25 -> 0.107, k = 2 0.82 -> 0.39, k = 3 2.09 ->
+// 1.01, k = 4 5.81 -> 3.47 (128x128 cells), k = 5 4.16 -> 2.11 (64x64).
+// Without the padded strides (kJacStride, kFaceStride, TS; k = 4, 64x64) 1.07,
+// with them 0.90.
 template <int Q, int WR, int WC>
 __host__ __device__ constexpr int condense_inv_aux() {  // doubles of J, later of one side's C R A^{-1}
   constexpr int P = Q * Q, M = 4 * P, T = 4 * Q;
-  return 32 * P > M * T ? 32 * P : M * T;
+  return kJacStride * P > M * (T + 2) ? kJacStride * P : M * (T + 2);
 }
 
-template <int Q, int WR, int WC, int MINB>
-__global__ void __launch_bounds__(32 * WR *WC, MINB)
+template <int Q, int WR, int WC, int DED, int MINB>
+__global__ void __launch_bounds__(32 * (WR * WC + DED), MINB)
     condense_inv_kernel(Geo g, const double *__restrict__ tab, Frozen fz, const double *__restrict__ u,
                         const double *__restrict__ r, double *XY, double *Cb, double *sf_out, double *contrib,
                         double *panels, int *redo, int *redo_count) {
-  using C = InvCfg<Q, WR, WC>;
-  constexpr int M = C::M, T = C::T, NR = 4 * T + 1, LDA = C::LDA;
+  using C = InvCfg<Q, WR, WC, DED>;
+  // TS: stride of C_s R_s A^{-1}; T + 2 is twice an odd number, so 16-byte
+  // stores with lanes over columns use all banks
+  constexpr int M = C::M, T = C::T, NR = 4 * T + 1, LDA = C::LDA, TS = T + 2;
   __shared__ CondenseInvShared<Q> sh;
   __shared__ __align__(16) double tiles[256];
   extern __shared__ __align__(16) double A[];
@@ -274,11 +283,11 @@ __global__ void __launch_bounds__(32 * WR *WC, MINB)
           v[2] += f * p1.x;
           v[3] += f * p1.y;
         }
-        const double *cb = sh.CB + (s * Q + jj) * 16;
+        const double *cb = sh.CB + (s * Q + jj) * kFaceStride;
         double o[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) o[c] = (cb[c] * v[0] + cb[c + 4] * v[1]) + (cb[c + 8] * v[2] + cb[c + 12] * v[3]);
-        double2 *dst = reinterpret_cast<double2 *>(aux + (size_t)col * T + 4 * jj);
+        double2 *dst = reinterpret_cast<double2 *>(aux + (size_t)col * TS + 4 * jj);
         dst[0] = make_double2(o[0], o[1]);
         dst[1] = make_double2(o[2], o[3]);
       }
@@ -292,7 +301,7 @@ __global__ void __launch_bounds__(32 * WR *WC, MINB)
 #pragma unroll
             for (int d = 0; d < 4; ++d) v[d] += f * p[d];
           }
-          const double *cb = sh.CB + t * 16;
+          const double *cb = sh.CB + t * kFaceStride;
 #pragma unroll
           for (int c = 0; c < 4; ++c)
             contrib[(size_t)e * 4 * T + 4 * t + c] =
@@ -303,7 +312,7 @@ __global__ void __launch_bounds__(32 * WR *WC, MINB)
       for (int t = threadIdx.x; t < T * T; t += blockDim.x) {
         const int row = t % T, jc = t / T;
         double x[4];
-        lift_row<Q>(sh.lift, aux + row, T, jc, x);
+        lift_row<Q>(sh.lift, aux + row, TS, jc, x);
         if (g.npan == 16) {
 #pragma unroll
           for (int o = 0; o < 4; ++o) panels[(((size_t)e * 16 + s * 4 + o) * T + jc) * T + row] = x[o];
@@ -610,11 +619,11 @@ static int sm_count_hdg() {
   return n;
 }
 
-template <int Q, int WR, int WC, int MINB>
+template <int Q, int WR, int WC, int DED, int MINB>
 static void launch_condense_inv(Ctx &c, const double *u, const double *r) {
-  using C = InvCfg<Q, WR, WC>;
+  using C = InvCfg<Q, WR, WC, DED>;
   constexpr size_t dyn = sizeof(double) * (size_t)(C::REGION + condense_inv_aux<Q, WR, WC>());
-  auto kern = condense_inv_kernel<Q, WR, WC, MINB>;
+  auto kern = condense_inv_kernel<Q, WR, WC, DED, MINB>;
   EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
   const int grid = std::min(c.n, sm_count_hdg() * MINB);
   kern<<<grid, C::THREADS, dyn, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, r, c.XY, c.Cb,
@@ -650,17 +659,23 @@ static void condense_redo(Ctx &c, const double *u, const double *r, int count) {
   launch_condensed_rhs(c);
 }
 
+// Warps per cell and cells per SM. One warp holds the tiles up to k = 2, four
+// at k = 3 and 4, with as many cells per SM as registers and shared memory allow: two
+// warps at k = 2 take 0.47 instead of 0.39 ms; k = 3 with four tile warps and
+// a fifth for the pivot blocks 1.19 instead of 1.01. At k = 5 one cell
+// fills the SM, and the warp for the pivot blocks pays: 2.11 against 2.24 ms (5
+// x 3 tile warps; 2 x 5 take 2.16). From k = 6 on a cell takes a cluster.
 void condense_launch(Ctx &c, const double *u, const double *r) {
   c.ensure_hdg();
   {
     ProfScope ps(c, EG_K_CONDENSE, 2);
     switch (c.q) {
-      case 1: launch_condense_inv<1, 1, 1, 16>(c, u, r); break;
-      case 2: launch_condense_inv<2, 1, 1, 16>(c, u, r); break;
-      case 3: launch_condense_inv<3, 1, 1, 10>(c, u, r); break;
-      case 4: launch_condense_inv<4, 2, 2, 4>(c, u, r); break;
-      case 5: launch_condense_inv<5, 2, 2, 2>(c, u, r); break;
-      case 6: launch_condense_inv<6, 3, 4, 1>(c, u, r); break;
+      case 1: launch_condense_inv<1, 1, 1, 0, 16>(c, u, r); break;
+      case 2: launch_condense_inv<2, 1, 1, 0, 16>(c, u, r); break;
+      case 3: launch_condense_inv<3, 1, 1, 0, 8>(c, u, r); break;
+      case 4: launch_condense_inv<4, 2, 2, 0, 4>(c, u, r); break;
+      case 5: launch_condense_inv<5, 2, 2, 0, 2>(c, u, r); break;
+      case 6: launch_condense_inv<6, 5, 3, 1, 1>(c, u, r); break;
       default: launch_condense_cluster(c, u, r);
     }
     EG_CUDA(cudaGetLastError());
