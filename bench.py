@@ -90,6 +90,9 @@ def algorithmic(w):
         "dg_apply": ("hbm", 8.0 * (2 * nu + 32 * n * p + 32 * nf * q)),
         "residual": ("hbm", 8.0 * (3 * nu + 6 * nf * q)),
         "pc_apply": ("hbm", 8.0 * (nf * t * t + 2 * nl) if w["form"] == "hdg" else 8.0 * (n * m * m + 2 * nu)),
+        # the one-kernel solve, per Krylov step: the Schur action, the block inverses
+        # and the new basis vector (the projection's reads of the basis are not counted)
+        "krylov": ("hbm", 8.0 * ((n * 16 * t * t if q >= 5 else n * m * 4 * t + 64 * n * q) + nf * t * t + 4 * nl)),
         "condense": ("fp64", n * (2.0 / 3.0 * m ** 3 + 2.0 * m * m * (4 * t + 1))),
         "dg_jacobi": ("fp64", n * (2.0 / 3.0 * m ** 3)),
     }
@@ -473,6 +476,7 @@ def run_ours(args, world, rank, local):
     ctx.lib.eg_profile_reset(ctx.h)
     ctx.lib.eg_profile_enable(ctx.h, 1)
     timed_updates(ctx, stepper, KP, world, ext)
+    krylov_prof = timed_updates.krylov
     prof = {}
     for i, name in enumerate(K_NAMES):
         import ctypes as C
@@ -537,8 +541,14 @@ def run_ours(args, world, rank, local):
     roofline = None
     fp64_peak = None
     dom_ms, dom_launch = prof[dominant]
-    ops_per = {"schur_apply": 2, "condense": 2}.get(dominant, 1)
-    nops = max(1, dom_launch // ops_per)
+    # operations behind a class's launches: a solve is one launch of many Krylov steps
+    nops_of = {"schur_apply": lambda cnt: cnt // 2, "condense": lambda cnt: cnt // 2,
+               "residual": lambda cnt: cnt // 2, "krylov": lambda cnt: krylov_prof if cnt else 0}
+
+    def operations(name, cnt):
+        return nops_of.get(name, lambda c: c)(cnt)
+
+    nops = max(1, operations(dominant, dom_launch))
     if dominant in alg:
         kind, units = alg[dominant]
         avg_s = dom_ms * 1e-3 / nops
@@ -558,14 +568,13 @@ def run_ours(args, world, rank, local):
                         "algorithmic_flops_per_launch": units, "avg_launch_ms": avg_s * 1e3,
                         "launches": nops,
                         "peak_source": "measured FP64 DGEMM (torch.matmul float64 4096^3) on this GPU"}
-    # second roofline line for the HBM-bound Schur apply (the matrix-free hot loop)
+    # the HBM-bound classes (the solve is the matrix-free hot loop)
     hbm_lines = {}
-    for name in ("schur_apply", "recover", "pc_apply", "residual", "dg_apply"):
+    for name in ("krylov", "schur_apply", "recover", "pc_apply", "residual", "dg_apply"):
         ms, cnt = prof[name]
-        # kernels per operation: the Schur action (panel GEMV + face combine) and
-        # the residual (face values, then the cell kernel) launch two
-        per = 2 if name in ("schur_apply", "residual") else 1
-        n_op = cnt // per
+        # the Schur action (panel GEMV + face combine) and the residual (face
+        # values, then the cell kernel) launch two kernels each
+        n_op = operations(name, cnt)
         if n_op and name in alg:
             avg_s = ms * 1e-3 / n_op
             ach = alg[name][1] / avg_s / 1e9
