@@ -59,9 +59,9 @@ enum eg_status {
   EG_ERR_UPDATE_EQUATION = 22,  /* "Independent recovered DG equation check failed" stepper.cpp:190 */
   EG_ERR_UPDATE_EQUIVALENCE = 23, /* "DG/HDG one-update equivalence failed" stepper.cpp:197 */
   EG_ERR_WAIT_LIMIT = 24,       /* a bounded device-side wait gave up: a dependency-driven block
-                                   ILU(0) factor or sweep, or a bulk copy of the DG block-Jacobi
-                                   record apply (no counterpart in the reference, whose factor and
-                                   sweeps are serial); the context stays usable */
+                                   ILU(0) factor or sweep, or a grid barrier of the one-launch
+                                   GMRES solve (no counterpart in the reference, which is serial);
+                                   the context stays usable */
   EG_ERR_CONTEXT_LOST = 25,     /* after a wait gave up, a bulk copy of the aborted sweep did not
                                    land within its own bound either: the context's device memory
                                    can no longer be trusted, every later call on it returns this
@@ -96,11 +96,8 @@ enum eg_slot {
   EG_SLOT_X = 7,       /* HDG responses X, n blocks of m x 4t column-major */
   EG_SLOT_Y = 8,       /* HDG particular responses y (nu) */
   EG_SLOT_PC_BLOCKS = 9, /* preconditioner blocks, column-major (count: eg_pc_size).
-                          block-jacobi: DG n*m*m, HDG nf*t*t; after eg_pc_factor(ctx, 1) HDG
-                          and DG with k <= 5 hold explicit inverses (DG column-major; for
-                          k = 3..5 the device keeps a Gauss-Jordan record and the
-                          download expands it into the inverses it applies), DG
-                          with k >= 6 packed pivoted LU.
+                          block-jacobi: DG n*m*m, HDG nf*t*t; after eg_pc_factor(ctx, 1) both
+                          hold explicit inverses.
                           block-ilu0: the BSR blocks of the ILU in FixedBlockILU order (rows
                           ascending, block columns ascending); after eg_pc_factor(ctx, 1) the
                           strictly lower blocks hold L, the others U (diagonal unfactored). */
@@ -452,9 +449,9 @@ long long eg_launch_count(const eg_ctx *ctx);
  * counterpart: the reference divides by each pivot). */
 int eg_check_pivot_reciprocal(const double *x, double *y, long long n);
 
-/* Test setting of the block ILU(0) device waits (no reference counterpart:
- * the reference's factor and sweeps are serial). limit_ns bounds every wait
- * of the factor and the sweeps (0 restores the default, 250 ms); starve != 0
+/* Test setting of the device waits (no reference counterpart: the reference
+ * is serial). limit_ns bounds every wait of the block ILU(0) factor and sweeps
+ * and of the one-launch GMRES solve (0 restores the default, 250 ms); starve != 0
  * makes every wait on another CTA unreachable, so that the next factor or
  * apply runs out its bound, returns EG_ERR_WAIT_LIMIT and leaves the context
  * usable. Applies to both forms' plans, including ones built later. */

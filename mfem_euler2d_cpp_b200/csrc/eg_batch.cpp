@@ -174,10 +174,10 @@ long long estimate_bytes(const eg_request &r) {
     d += n * m * (4 * t + 1) + n * 4 * q * 17 + n * 4 * t + n * (q >= 5 ? 16 : 4) * t * t + 4 * nl + nf * t * t +
          nf * t / 2;
     if (r.precision == EG_PRECISION_MIXED) d += (n * m * 4 * t + nf * t * t + nl * (R + 9) + n * 4 * t) / 2;
-    if (r.precond == EG_PC_BLOCK_ILU0) d += 8 * nf * t * t + n * 16 * t * t;
+    if (r.precond == EG_PC_BLOCK_ILU0) d += 8 * nf * t * t + n * 16 * t * t + 3 * nl;  // 2 nl: hand-over words
   } else {
     d += n * m * m + n * m / 2;
-    if (r.precond == EG_PC_BLOCK_ILU0) d += 6 * n * m * m;
+    if (r.precond == EG_PC_BLOCK_ILU0) d += 6 * n * m * m + 3 * nu;
   }
   return d * 8 + d * 8 / 50;  // 2% for small tables and workspaces
 }

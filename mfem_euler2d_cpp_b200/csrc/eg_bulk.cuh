@@ -1,7 +1,7 @@
 // mbarrier-completed bulk copies (cp.async.bulk, global -> this CTA's own
-// shared memory, one destination CTA) shared by the block ILU(0) sweeps
-// (eg_ilu.cu) and the DG block-Jacobi record apply (eg_dginv.cu). Every wait
-// is bounded by a poll count chosen by the caller. Not part of the C-ABI.
+// shared memory, one destination CTA) of the block ILU(0) sweeps for blocks of
+// at most 36 (eg_ilu.cu). Every wait is bounded by a poll count chosen by the
+// caller. Not part of the C-ABI.
 #pragma once
 
 namespace eg {

@@ -124,7 +124,6 @@ struct SweepArgs {
   unsigned long long *progress;
   int *abort, *err;
   unsigned long long tag;
-  int staged;        // stage up to kStageBlocks blocks per row in shared memory
   unsigned long long limit_ns;  // bound of every wait
   int starve;        // test setting: waits on other CTAs can never be met
   uint4 *slots;      // small blocks: the rows' values for other CTAs
@@ -137,26 +136,21 @@ struct SweepArgs {
 // CTA keep W rows and their block copies in flight. A finished row goes to a
 // shared-memory ring (read by later rows of the same CTA) and to global
 // memory; the CTA's own count is published first, then, off the local chain,
-// the release of the global counter that other CTAs poll.
+// the release of the global counter that other CTAs poll. For blocks above
+// kStageMaxB, read from global memory; smaller ones take the kernel below.
 template <int S, bool BACK>
 __global__ void __launch_bounds__(256, 1) ilu_sweep_kernel(SweepArgs a) {
   extern __shared__ __align__(128) double smem[];
   __shared__ unsigned done_local;
-  __shared__ __align__(8) unsigned long long bars[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
   const int g = blockIdx.x, B = a.B;
   const size_t BB = (size_t)B * B;
   const int p0 = a.slot_ptr[g], nslots = a.slot_ptr[g + 1] - p0;
-  const size_t stage_doubles = a.staged ? kStageBlocks * BB : 0;
-  double *stage = smem + (size_t)warp * stage_doubles;
-  double *vb = smem + (size_t)W * stage_doubles + (size_t)warp * 32 * S;
-  double *ring = smem + (size_t)W * (stage_doubles + 32 * S);
+  double *vb = smem + (size_t)warp * 32 * S;
+  double *ring = smem + (size_t)W * 32 * S;
   if (threadIdx.x == 0) done_local = 0;
-  if (a.staged && lane == 0) mbar_init(&bars[warp]);
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
   volatile unsigned *dl = &done_local;
-  unsigned phase = 0;
   int4 nm = make_int4(0, 0, 0, 0);
   int2 nd[kMaxDeps];
   auto fetch = [&](int slot) {
@@ -173,32 +167,11 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_kernel(SweepArgs a) {
 #pragma unroll
     for (int k = 0; k < kMaxDeps; ++k) dep[k] = nd[k];
     fetch(slot + W);  // the next row's schedule is in flight during this row
-    const int nst = a.staged ? min(ne, BACK ? kStageBlocks - 1 : kStageBlocks) : 0;
-    const bool copy = a.staged && (nst > 0 || BACK);
-    if (copy && lane == 0) {
-      const unsigned bytes = (unsigned)(sizeof(double) * BB * (nst + (BACK ? 1 : 0)));
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_expect(&bars[warp], bytes);
-      if (nst) bulk_load(stage, a.data + (size_t)e0 * BB, (unsigned)(sizeof(double) * BB * nst), &bars[warp]);
-      if (BACK) bulk_load(stage + (size_t)nst * BB, a.dinv + (size_t)i * BB, (unsigned)(sizeof(double) * BB),
-                          &bars[warp]);
-    }
     double acc[S];
 #pragma unroll
     for (int s = 0; s < S; ++s) {
       const int r = lane + 32 * s;
       acc[s] = r < B ? __ldcg(a.in + (size_t)i * B + r) : 0.;
-    }
-    if (copy) {
-      if (!mbar_wait(&bars[warp], phase, kCopySpinLimit)) {
-        give_up(a.abort, a.err);
-        // let the copy land before the CTA can exit; if even the longer drain
-        // bound runs out, the copy may still write this CTA's shared memory:
-        // err[2] tells the host that the context can no longer be trusted
-        if (!mbar_wait(&bars[warp], phase, kDrainSpinLimit) && lane == 0) atomicExch(a.err + 2, 1);
-        return;
-      }
-      phase ^= 1u;
     }
     bool ok = true;
 #pragma unroll
@@ -214,7 +187,7 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_kernel(SweepArgs a) {
           const double *src = ring + (size_t)(js & (a.ring - 1)) * B;
           for (int r = lane; r < B; r += 32) vb[r] = in_ring ? src[r] : __ldcg(a.out + (size_t)j * B + r);
           __syncwarp();
-          const double *A = k < nst ? stage + (size_t)k * BB : a.data + (size_t)(e0 + k) * BB;
+          const double *A = a.data + (size_t)(e0 + k) * BB;
 #pragma unroll
           for (int s = 0; s < S; ++s) {
             const int r = lane + 32 * s;
@@ -240,7 +213,7 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_kernel(SweepArgs a) {
         if (r < B) vb[r] = acc[s];
       }
       __syncwarp();
-      const double *Di = a.staged ? stage + (size_t)nst * BB : a.dinv + (size_t)i * BB;
+      const double *Di = a.dinv + (size_t)i * BB;
 #pragma unroll
       for (int s = 0; s < S; ++s) {
         const int r = lane + 32 * s;
@@ -303,7 +276,7 @@ __device__ __forceinline__ bool get_slot(const uint4 *p, unsigned ep, double &v)
 // A row's products are four partial sums each, unrolled; its neighbours' rows
 // in other CTAs are polled together and folded in before its own CTA's.
 // 48x48 Q4, forward and backward sweep: 1190 us with the counters and run-time
-// block sizes of the kernel above, see the launch table in the driver below.
+// block sizes of the kernel above, 430 here.
 template <int B, bool BACK>
 __global__ void __launch_bounds__(256, 1) ilu_sweep_small_kernel(SweepArgs a) {
   constexpr int S = (B + 31) / 32, BB = B * B;
@@ -597,7 +570,8 @@ __global__ void __launch_bounds__(256, 1) ilu_factor_kernel(FactorArgs a) {
 // block is inverted by one warp in registers, a row per lane: Gauss-Jordan in
 // place with row pivoting, no barrier in its steps. One CTA per row as there;
 // the chain of rows bounds it, so what counts is the latency of a row.
-// 48x48 Q4: 16.3 ms with the kernel above, see the driver below.
+// 48x48 Q4: 16.3 ms with the kernel above, 5.8 here. That one keeps B = 36,
+// whose rows do not fit one warp's lanes.
 template <int B>
 __global__ void __launch_bounds__(512, 1) ilu_factor_small_kernel(FactorArgs a) {
   constexpr int BB = B * B;
@@ -843,7 +817,6 @@ int sweep_occupancy(int block, size_t smem) {
 }
 int sweep_occupancy_dispatch(int S, int block, size_t smem) {
   switch (S) {
-    case 1: return sweep_occupancy<1>(block, smem);
     case 2: return sweep_occupancy<2>(block, smem);
     case 3: return sweep_occupancy<3>(block, smem);
     case 4: return sweep_occupancy<4>(block, smem);
@@ -1121,7 +1094,6 @@ void sweep(Ctx &c, IluPlan &P, const double *in, double *out) {
   a.abort = P.abort;
   a.err = c.derr;
   a.tag = (unsigned long long)(++P.epoch) << 32;
-  a.staged = P.staged;
   a.limit_ns = P.wait_limit_ns;
   a.starve = P.starve;
   a.slots = static_cast<uint4 *>(P.slots);
@@ -1133,7 +1105,8 @@ void sweep(Ctx &c, IluPlan &P, const double *in, double *out) {
       return;
     }
   }
-  launch_coop(ilu_sweep_kernel<S, BACK>, P.grid_sweep, 32 * P.sweep_warps, P.sweep_smem, c.stream, a);
+  if constexpr (S >= 2)
+    launch_coop(ilu_sweep_kernel<S, BACK>, P.grid_sweep, 32 * P.sweep_warps, P.sweep_smem, c.stream, a);
 }
 
 template <bool BACK>
