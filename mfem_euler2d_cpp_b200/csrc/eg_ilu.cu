@@ -276,7 +276,7 @@ __device__ __forceinline__ bool get_slot(const uint4 *p, unsigned ep, double &v)
 // A row's products are four partial sums each, unrolled; its neighbours' rows
 // in other CTAs are polled together and folded in before its own CTA's.
 // 48x48 Q4, forward and backward sweep: 1190 us with the counters and run-time
-// block sizes of the kernel above, 430 here.
+// block sizes of the kernel above, 417 here.
 template <int B, bool BACK>
 __global__ void __launch_bounds__(256, 1) ilu_sweep_small_kernel(SweepArgs a) {
   constexpr int S = (B + 31) / 32, BB = B * B;
@@ -378,30 +378,45 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_small_kernel(SweepArgs a) {
     }
     if (!ok) return;
     __syncwarp();
-    const auto product = [&](const double *A, const double *v, double sign) {
+    // the lane's rows of a block, read before the vector is there
+    double ar[S][B];
+    const auto load_block = [&](const double *A) {
 #pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int r = lane + 32 * s;
-        if (r < B) {
-          double t[4] = {0., 0., 0., 0.};
+      for (int s = 0; s < S; ++s)
 #pragma unroll
-          for (int cc = 0; cc < B; cc += 4)
+        for (int cc = 0; cc < B; ++cc) ar[s][cc] = lane + 32 * s < B ? A[cc * B + lane + 32 * s] : 0.;
+    };
+    const auto product = [&](const double *v, double sign) {
+      double t[S][4];
 #pragma unroll
-            for (int k4 = 0; k4 < 4; ++k4) t[k4] = fma(A[(cc + k4) * B + r], v[cc + k4], t[k4]);
-          acc[s] = fma(sign, (t[0] + t[1]) + (t[2] + t[3]), acc[s]);
+      for (int s = 0; s < S; ++s) t[s][0] = t[s][1] = t[s][2] = t[s][3] = 0.;
+#pragma unroll
+      for (int cc = 0; cc < B; cc += 4) {
+        const double2 a = *reinterpret_cast<const double2 *>(v + cc), b = *reinterpret_cast<const double2 *>(v + cc + 2);
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+          t[s][0] = fma(ar[s][cc], a.x, t[s][0]);
+          t[s][1] = fma(ar[s][cc + 1], a.y, t[s][1]);
+          t[s][2] = fma(ar[s][cc + 2], b.x, t[s][2]);
+          t[s][3] = fma(ar[s][cc + 3], b.y, t[s][3]);
         }
       }
+#pragma unroll
+      for (int s = 0; s < S; ++s) acc[s] = fma(sign, (t[s][0] + t[s][1]) + (t[s][2] + t[s][3]), acc[s]);
     };
 #pragma unroll
     for (int k = 0; k < kMaxDeps; ++k)
-      if (k < ne && (dep[k].x >> kOwnerShift) != g)
-        product(k < nst ? stage + (size_t)k * BB : a.data + (size_t)(e0 + k) * BB, vb + k * B, -1.);
+      if (k < ne && (dep[k].x >> kOwnerShift) != g) {
+        load_block(k < nst ? stage + (size_t)k * BB : a.data + (size_t)(e0 + k) * BB);
+        product(vb + k * B, -1.);
+      }
     // the CTA's own rows, the ones finished first in front
 #pragma unroll
     for (int k0 = 0; k0 < kMaxDeps; ++k0) {
       const int k = BACK ? kMaxDeps - 1 - k0 : k0;
       if (k < ne && (dep[k].x >> kOwnerShift) == g && ok) {
         const int js = dep[k].x & kSlotMask;
+        load_block(k < nst ? stage + (size_t)k * BB : a.data + (size_t)(e0 + k) * BB);
         ok = wait_local(dl, (unsigned)js + 1, a.abort, a.err, a.limit_ns);
         if (ok) {
           __threadfence_block();
@@ -411,7 +426,7 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_small_kernel(SweepArgs a) {
             __syncwarp();
             v = vb + k * B;
           }
-          product(k < nst ? stage + (size_t)k * BB : a.data + (size_t)(e0 + k) * BB, v, -1.);
+          product(v, -1.);
         }
       }
     }
@@ -421,22 +436,30 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_small_kernel(SweepArgs a) {
 #pragma unroll
       for (int s = 0; s < S; ++s)
         if (lane + 32 * s < B) vb[lane + 32 * s] = acc[s];
+      load_block(stage + (size_t)nst * BB);
       __syncwarp();
 #pragma unroll
       for (int s = 0; s < S; ++s) acc[s] = 0.;
-      product(stage + (size_t)nst * BB, vb, 1.);
+      product(vb, 1.);
     }
     double *rs = ring + (size_t)(slot & (a.ring - 1)) * B;
 #pragma unroll
     for (int s = 0; s < S; ++s) {
       const int r = lane + 32 * s;
+      if (r < B) rs[r] = acc[s];
+    }
+    __threadfence_block();
+    // behind the fence, which would wait for them: other CTAs check the words
+    // themselves, and this CTA reads `out` only for rows that left the ring,
+    // whose warp has fenced again for its next row since (ring >= 4 W)
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      const int r = lane + 32 * s;
       if (r < B) {
-        rs[r] = acc[s];
         put_slot(a.slots + (size_t)i * B + r, acc[s], a.epoch);
         a.out[(size_t)i * B + r] = acc[s];
       }
     }
-    __threadfence_block();
     __syncwarp();
     int pub = 1;
     if (lane == 0) {
@@ -984,7 +1007,7 @@ void build_plan(Ctx &c, int form) {
                              (size_t)P.ring * P.B);
   };
   while (W > 1 && sweep_smem(W) > kSweepSmemBudget) --W;
-  if (P.ring < 2 * W) fail(EG_ERR_INVALID, "block ILU ring too small");
+  if (P.ring < (P.staged ? 4 : 2) * W) fail(EG_ERR_INVALID, "block ILU ring too small");
   P.sweep_warps = W;
   P.sweep_smem = sweep_smem(W);
   P.factor_smem = !P.staged ? 0
