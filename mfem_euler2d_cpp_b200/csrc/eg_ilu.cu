@@ -32,7 +32,7 @@
 #include <vector>
 
 #include "eg_bulk.cuh"
-#include "eg_cellmat.cuh"
+#include "eg_cellinv.cuh"
 #include "eg_internal.h"
 
 namespace eg {
@@ -43,6 +43,7 @@ constexpr unsigned kDrainSpinLimit = 1u << 24;  // abort path: let an issued cop
 constexpr int kStageBlocks = 4;             // blocks staged per warp and row
 constexpr int kStageMaxB = 36;              // larger blocks are read from global memory
 constexpr size_t kSweepSmemBudget = 210 * 1024;
+constexpr size_t kFactorSmemBudget = 220 * 1024;
 constexpr size_t kRingBytes = 48 * 1024;    // shared-memory ring of finished rows per CTA
 
 // ------------------------------------------------------------ sync helpers
@@ -473,6 +474,7 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_small_kernel(SweepArgs a) {
 // ----------------------------------------------------------- factor kernel
 struct FactorArgs {
   int B, maxrow, maxupd, maxl, maxtot;
+  int ahead;          // small blocks: the next row's blocks have a buffer of their own
   const int *slot_ptr;
   const int4 *meta;   // forward schedule: (row, first lower entry, lower count)
   const int2 *deps;
@@ -586,35 +588,72 @@ __global__ void __launch_bounds__(256, 1) ilu_factor_kernel(FactorArgs a) {
   }
 }
 
+// One 8x8 tile of sign X Y added to (d0, d1), B x B blocks column-major in
+// shared memory, zero beyond B. Free of bank conflicts: B % 8 == 4, or the rows
+// of a tile are next to each other.
+template <int B>
+__device__ __forceinline__ void block_tile(double &d0, double &d1, const double *X, const double *Y, int tr, int tc,
+                                           double sign) {
+  const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3, r = 8 * tr + gq, c = 8 * tc + gq;
+#pragma unroll
+  for (int s = 0; s < B; s += 4)
+    dmma_m8n8k4(d0, d1, r < B ? sign * X[(s + tq) * B + r] : 0., c < B ? Y[c * B + s + tq] : 0.);
+}
+
 // Factor for blocks of at most 32 (every HDG degree below 8): the arithmetic
-// of ilu_factor_kernel with the block size known at compile time. A row's
-// blocks are read before its neighbours are waited for, all blocks of the
-// neighbours (inverse diagonals and retained U) in one round, and the diagonal
-// block is inverted by one warp in registers, a row per lane: Gauss-Jordan in
-// place with row pivoting, no barrier in its steps. One CTA per row as there;
-// the chain of rows bounds it, so what counts is the latency of a row.
-// 48x48 Q4: 16.3 ms with the kernel above, 5.8 here. That one keeps B = 36,
-// whose rows do not fit one warp's lanes.
+// of ilu_factor_kernel with the block size known at compile time. One CTA per
+// row as there; the chain of rows bounds it, so what counts is the latency of a
+// row. Its schedule and (where they fit twice) its blocks are fetched while the
+// row before inverts its diagonal block, all blocks of its neighbours (inverse
+// diagonals and retained U) are read in one round, products run on the FP64
+// tensor pipe, and the diagonal block is inverted by one warp in registers, a
+// row per lane: Gauss-Jordan in place with row pivoting, no barrier in its
+// steps, the search for the next pivot under the other columns' update.
+// 48x48 Q4: 16.3 ms with the kernel above, 3.6 here (5.8 with a row fetched when
+// its turn came and products by FMAs out of shared memory). The kernel above
+// keeps B = 36, whose rows do not fit one warp's lanes.
 template <int B>
 __global__ void __launch_bounds__(512, 1) ilu_factor_small_kernel(FactorArgs a) {
-  constexpr int BB = B * B;
+  constexpr int BB = B * B, MT = (B + 7) / 8, TILES = MT * MT;
   extern __shared__ __align__(16) double fsm[];
   __shared__ int stop;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ int4 s_row[2];  // row, lower count, first entry, entries
+  __shared__ int2 s_dep[2][kMaxDeps], s_upd[2][kMaxDeps * kMaxDeps];  // updates: (target entry in the row, U entry)
+  __shared__ int s_ptr[2][kMaxDeps + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int g = blockIdx.x, p0 = a.slot_ptr[g], nslots = a.slot_ptr[g + 1] - p0;
-  double *rowblk = fsm;                              // the row's blocks (maxrow)
-  double *Dk = rowblk + (size_t)a.maxrow * BB;       // U_kk^{-1} of the lower neighbours (maxl)
-  double *Ub = Dk + (size_t)a.maxl * BB;             // their retained U_kj (maxtot)
+  double *rows = fsm;                                      // a.ahead + 1 buffers for a row's blocks (maxrow)
+  double *Dk = rows + (size_t)(a.ahead + 1) * a.maxrow * BB;  // U_kk^{-1} of the lower neighbours (maxl)
+  double *Ub = Dk + (size_t)a.maxl * BB;                   // their retained U_kj (maxtot)
   double *Lt = Ub + (size_t)a.maxtot * BB;
-  for (int slot = 0; slot < nslots; ++slot) {
+  const auto row_blocks = [&](int slot) { return rows + (size_t)(slot & a.ahead) * a.maxrow * BB; };
+  const auto load_row = [&](int slot, int rb, int nb, int t, int nt) {
+    const double2 *src = reinterpret_cast<const double2 *>(a.data + (size_t)rb * BB);
+    double2 *dst = reinterpret_cast<double2 *>(row_blocks(slot));
+    for (int o = t; o < nb * BB / 2; o += nt) dst[o] = src[o];
+  };
+  // the schedule of a row, by threads t of nt >= 64
+  const auto fetch = [&](int slot, int t, int nt) {
+    const int buf = slot & 1;
     const int4 m = a.meta[p0 + slot];
-    const int i = m.x, nl = m.z, rb = a.row[i], re = a.row[i + 1], di = a.diag[i];
-    const int u0 = a.upd_ptr[rb], ntot = a.upd_ptr[di] - u0;
-    for (int o = threadIdx.x; o < (re - rb) * BB; o += blockDim.x) rowblk[o] = a.data[(size_t)rb * BB + o];
+    const int rb = a.row[m.x], nb = a.row[m.x + 1] - rb, u0 = a.upd_ptr[rb], ntot = a.upd_ptr[rb + m.z] - u0;
+    if (t == 0) s_row[buf] = make_int4(m.x, m.z, rb, nb);
+    if (t < m.z) s_dep[buf][t] = a.deps[(size_t)(p0 + slot) * kMaxDeps + t];
+    if (t <= m.z) s_ptr[buf][t] = a.upd_ptr[rb + t] - u0;
+    if (t < ntot) s_upd[buf][t] = make_int2(a.upd[2 * (u0 + t)] - rb, a.upd[2 * (u0 + t) + 1]);
+    if (a.ahead) load_row(slot, rb, nb, t, nt);
+  };
+  if (nslots > 0) fetch(0, threadIdx.x, blockDim.x);
+  __syncthreads();
+  for (int slot = 0; slot < nslots; ++slot) {
+    const int buf = slot & 1;
+    const int i = s_row[buf].x, nl = s_row[buf].y, rb = s_row[buf].z, nb = s_row[buf].w;
+    double *rowblk = row_blocks(slot);
+    if (!a.ahead) load_row(slot, rb, nb, threadIdx.x, blockDim.x);
     if (threadIdx.x == 0) {
       int ok = 1;
       for (int k = 0; k < nl && ok; ++k) {
-        const int2 d = a.deps[(size_t)(p0 + slot) * kMaxDeps + k];
+        const int2 d = s_dep[buf][k];
         const int owner = d.x >> kOwnerShift, js = d.x & kSlotMask;
         if (owner != g)
           ok = wait_progress(a.progress + owner, need(a.tag, js, a.starve), a.abort, a.err, a.limit_ns);
@@ -623,50 +662,59 @@ __global__ void __launch_bounds__(512, 1) ilu_factor_small_kernel(FactorArgs a) 
     }
     __syncthreads();
     if (stop) return;
-    for (int o = threadIdx.x; o < (nl + ntot) * BB; o += blockDim.x) {
-      const int blk = o / BB, r = o % BB;
-      Dk[blk < nl ? o : (a.maxl - nl) * BB + o] =
-          blk < nl ? __ldcg(a.dinv + (size_t)a.deps[(size_t)(p0 + slot) * kMaxDeps + blk].y * BB + r)
-                   : __ldcg(a.data + (size_t)a.upd[2 * (u0 + blk - nl) + 1] * BB + r);
+    const int ntot = s_ptr[buf][nl];
+    for (int o = threadIdx.x; o < (nl + ntot) * (BB / 2); o += blockDim.x) {
+      const int blk = o / (BB / 2), e = o % (BB / 2);
+      const double *src = blk < nl ? a.dinv + (size_t)s_dep[buf][blk].y * BB
+                                   : a.data + (size_t)s_upd[buf][blk - nl].y * BB;
+      double *dst = blk < nl ? Dk + (size_t)blk * BB : Ub + (size_t)(blk - nl) * BB;
+      reinterpret_cast<double2 *>(dst)[e] = __ldcg(reinterpret_cast<const double2 *>(src) + e);
     }
     __syncthreads();
-    const auto dot = [](const double *A, const double *C) {  // row of A (stride B) times a column of C
-      double t[4] = {0., 0., 0., 0.};
-#pragma unroll
-      for (int s = 0; s < B; s += 4)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) t[k] = fma(A[(s + k) * B], C[s + k], t[k]);
-      return (t[0] + t[1]) + (t[2] + t[3]);
-    };
-    for (int ik = rb; ik < di; ++ik) {
-      const int v0 = a.upd_ptr[ik], nu = a.upd_ptr[ik + 1] - v0;
-      double *Aik = rowblk + (size_t)(ik - rb) * BB;
-      const double *D = Dk + (size_t)(ik - rb) * BB;
-      for (int o = threadIdx.x; o < BB; o += blockDim.x) Lt[o] = dot(Aik + o % B, D + (o / B) * B);
-      __syncthreads();
-      for (int o = threadIdx.x; o < (nu + 1) * BB; o += blockDim.x) {
-        const int uu = o / BB - 1, r = o % BB;
-        if (uu < 0)
-          Aik[r] = Lt[r];
-        else
-          rowblk[(size_t)(a.upd[2 * (v0 + uu)] - rb) * BB + r] -=
-              dot(Lt + r % B, Ub + (size_t)(v0 - u0 + uu) * BB + (r / B) * B);
+    const int gq = lane >> 2, tq = lane & 3;
+    for (int k = 0; k < nl; ++k) {
+      const int v0 = s_ptr[buf][k], nu = s_ptr[buf][k + 1] - v0;
+      double *Aik = rowblk + (size_t)k * BB;
+      for (int t = warp; t < TILES; t += nwarps) {
+        const int tr = t % MT, tc = t / MT, r = 8 * tr + gq, c = 8 * tc + 2 * tq;
+        double d0 = 0., d1 = 0.;
+        block_tile<B>(d0, d1, Aik, Dk + (size_t)k * BB, tr, tc, 1.);
+        if (r < B && c < B) {  // c + 1 too: B is even
+          Lt[c * B + r] = d0;
+          Lt[(c + 1) * B + r] = d1;
+        }
       }
+      __syncthreads();
+      for (int t = warp; t < nu * TILES; t += nwarps) {
+        const int uu = v0 + t / TILES, tr = t % MT, tc = t % TILES / MT, r = 8 * tr + gq, c = 8 * tc + 2 * tq;
+        double *T = rowblk + (size_t)s_upd[buf][uu].x * BB + c * B + r;
+        const bool in = r < B && c < B;
+        double d0 = in ? T[0] : 0., d1 = in ? T[B] : 0.;
+        block_tile<B>(d0, d1, Lt, Ub + (size_t)uu * BB, tr, tc, -1.);
+        if (in) {
+          T[0] = d0;
+          T[B] = d1;
+        }
+      }
+      for (int o = threadIdx.x; o < BB; o += blockDim.x) Aik[o] = Lt[o];
       __syncthreads();
     }
     if (warp == 0) {
-      const double *Ad = rowblk + (size_t)(di - rb) * BB;
+      const double *Ad = rowblk + (size_t)nl * BB;
       double w[B];
 #pragma unroll
       for (int c = 0; c < B; ++c) w[c] = lane < B ? Ad[c * B + lane] : 0.;
       bool un = lane < B, singular = false;
       int pos = 0, mycol = 0;  // the step whose pivot row this lane is; the pivot row of step `lane`
+      const auto search = [&](double x) {
+        // largest magnitude (within 2^-15), first row on ties
+        const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+        const unsigned key = (un && hi < 0x7ff00000u) ? ((hi & ~31u) | (unsigned)(31 - lane)) : 0u;
+        return __reduce_max_sync(0xffffffffu, key);
+      };
+      unsigned mb = search(w[0]);
 #pragma unroll
       for (int k = 0; k < B; ++k) {
-        // largest magnitude (within 2^-15), first row on ties
-        const unsigned hi = (unsigned)__double2hiint(w[k]) & 0x7fffffffu;
-        const unsigned key = (un && hi < 0x7ff00000u) ? ((hi & ~31u) | (unsigned)(31 - lane)) : 0u;
-        const unsigned mb = __reduce_max_sync(0xffffffffu, key);
         singular = singular || (mb >> 5) == 0u;
         const int p = 31 - (int)(mb & 31u);
         const bool me = lane == p;
@@ -675,11 +723,12 @@ __global__ void __launch_bounds__(512, 1) ilu_factor_small_kernel(FactorArgs a) 
         pos = me ? k : pos;
         un = un && !me;
 #pragma unroll
-        for (int c = 0; c < B; ++c)
-          if (c != k) {
-            const double v = __shfl_sync(0xffffffffu, w[c], p) * ip;
-            w[c] = me ? v : fma(-l, v, w[c]);
-          }
+        for (int c0 = 1; c0 < B; ++c0) {
+          const int c = (k + c0) % B;  // the next pivot's column first
+          const double v = __shfl_sync(0xffffffffu, w[c], p) * ip;
+          w[c] = me ? v : fma(-l, v, w[c]);
+          if (c0 == 1 && k + 1 < B) mb = search(w[c]);
+        }
         w[k] = me ? ip : -l * ip;
       }
       if (singular && lane == 0) raise_err(a.err, DERR_SINGULAR_ILU);
@@ -690,7 +739,10 @@ __global__ void __launch_bounds__(512, 1) ilu_factor_small_kernel(FactorArgs a) 
         if (lane < B) Di[col * B + pos] = w[c];
       }
     } else {
-      for (int o = threadIdx.x - 32; o < (re - rb) * BB; o += blockDim.x - 32) a.data[(size_t)rb * BB + o] = rowblk[o];
+      double2 *dst = reinterpret_cast<double2 *>(a.data + (size_t)rb * BB);
+      for (int o = threadIdx.x - 32; o < nb * BB / 2; o += blockDim.x - 32)
+        dst[o] = reinterpret_cast<const double2 *>(rowblk)[o];
+      if (slot + 1 < nslots) fetch(slot + 1, threadIdx.x - 32, blockDim.x - 32);
     }
     __threadfence();
     __syncthreads();
@@ -1010,9 +1062,14 @@ void build_plan(Ctx &c, int form) {
   if (P.ring < (P.staged ? 4 : 2) * W) fail(EG_ERR_INVALID, "block ILU ring too small");
   P.sweep_warps = W;
   P.sweep_smem = sweep_smem(W);
-  P.factor_smem = !P.staged ? 0
-                  : sizeof(double) * BB * (size_t)(factor_small(P.B) ? P.maxrow + P.maxl + P.maxtot + 1
-                                                                     : P.maxrow + P.maxupd + 4);
+  const auto factor_smem = [&](int row_buffers) {
+    return sizeof(double) * BB * (size_t)(row_buffers * P.maxrow + P.maxl + P.maxtot + 1);
+  };
+  P.ahead = factor_small(P.B) && factor_smem(2) <= kFactorSmemBudget ? 1 : 0;
+  P.factor_smem = !P.staged          ? 0
+                  : factor_small(P.B) ? factor_smem(P.ahead + 1)
+                                      : sizeof(double) * BB * (size_t)(P.maxrow + P.maxupd + 4);
+  if (P.staged && P.maxtot > kMaxDeps * kMaxDeps) fail(EG_ERR_INVALID, "block ILU row too long");
   const int occ = std::min(P.staged ? small_sweep_occupancy(P.B, 32 * W, P.sweep_smem)
                                     : sweep_occupancy_dispatch(S, 32 * W, P.sweep_smem),
                            factor_occupancy(P.B, P.staged != 0, P.factor_smem));
@@ -1173,6 +1230,7 @@ void factor_launch(Ctx &c, IluPlan &P) {
   a.limit_ns = P.wait_limit_ns;
   a.starve = P.starve;
   a.maxl = P.maxl;
+  a.ahead = P.ahead;
   a.maxtot = P.maxtot;
   if (SMEM && factor_small(P.B)) {
     EG_ILU_SMALL(P.B, if constexpr (BS <= 32)

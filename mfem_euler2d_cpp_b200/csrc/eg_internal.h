@@ -134,7 +134,7 @@ constexpr unsigned long long kIluWaitLimitNs = 250ull * 1000 * 1000;
 // the factored diagonal blocks. Built on first use (eg_ilu.cu).
 struct IluPlan {
   bool built = false;
-  int rows = 0, B = 0, nnzb = 0, chunk = 0, chunks = 0, maxl = 0, maxu = 0, maxtot = 0;
+  int rows = 0, B = 0, nnzb = 0, chunk = 0, chunks = 0, maxl = 0, maxu = 0, maxtot = 0, ahead = 0;
   int *row = nullptr, *col = nullptr, *diag = nullptr, *erow = nullptr;
   int *upd_ptr = nullptr, *upd = nullptr;        // per entry: (target, upper) pairs
   int *fill_ptr = nullptr, *fill_src = nullptr;  // per entry: fill contributions
