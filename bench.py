@@ -62,9 +62,9 @@ K_NAMES = ["residual", "dg_apply", "dg_jacobi", "condense", "schur_apply", "reco
 
 
 # DRAM bytes (read + write) per cell of one launch, from one ncu capture of the
-# kernel on a 64x64 mesh of the same degree (profiles/condense_gj2_q4_64x64.txt,
+# kernel on a 64x64 mesh of the same degree (profiles/condense_inv_q4_64x64.txt,
 # profiles/panel_gemv_q4_64x64.txt); per-launch traffic grows with the cell count.
-NCU_TRAFFIC_PER_CELL = {("condense", 4): 512.70e6 / 4096, ("schur_apply", 4): 216.24e6 / 4096}
+NCU_TRAFFIC_PER_CELL = {("condense", 4): 440.45e6 / 4096, ("schur_apply", 4): 216.24e6 / 4096}
 
 
 def traffic(name, w):

@@ -659,12 +659,12 @@ static void condense_redo(Ctx &c, const double *u, const double *r, int count) {
   launch_condensed_rhs(c);
 }
 
-// Warps per cell and cells per SM. One warp holds the tiles up to k = 2, four
-// at k = 3 and 4, with as many cells per SM as registers and shared memory allow: two
-// warps at k = 2 take 0.47 instead of 0.39 ms; k = 3 with four tile warps and
-// a fifth for the pivot blocks 1.19 instead of 1.01. At k = 5 one cell
-// fills the SM, and the warp for the pivot blocks pays: 2.11 against 2.24 ms (5
-// x 3 tile warps; 2 x 5 take 2.16). From k = 6 on a cell takes a cluster.
+// Warps per cell and cells per SM: one warp holds the tiles up to k = 2, four
+// at k = 3 and 4, with as many cells per SM as registers and shared memory
+// allow (two warps at k = 2: 0.47 instead of 0.39 ms; four and one for the
+// pivot blocks at k = 3: 1.19 instead of 1.01). At k = 5 one cell fills the SM,
+// and the warp for the pivot blocks pays: 2.11 against 2.24 ms (2 x 5 tile warps
+// instead of 5 x 3: 2.16). From k = 6 on a cell takes a cluster.
 void condense_launch(Ctx &c, const double *u, const double *r) {
   c.ensure_hdg();
   {
