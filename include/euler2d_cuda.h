@@ -457,6 +457,12 @@ int eg_check_pivot_reciprocal(const double *x, double *y, long long n);
  * usable. Applies to both forms' plans, including ones built later. */
 int eg_set_ilu_wait(eg_ctx *ctx, unsigned long long limit_ns, int starve);
 
+/* Test setting of the device allocations (no reference counterpart): the nth
+ * allocation of the context from now on (nth = 1: the next one) is refused as
+ * if the device had no memory left, and its call returns EG_ERR_OUT_OF_MEMORY;
+ * the ones after it succeed again. 0: none. */
+int eg_set_alloc_failure(eg_ctx *ctx, int nth);
+
 #ifdef __cplusplus
 }
 #endif

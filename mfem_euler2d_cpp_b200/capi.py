@@ -154,6 +154,7 @@ def load() -> C.CDLL:
         "eg_profile_query": (C.c_int, [vp, C.c_int, _DP, C.POINTER(C.c_longlong)]),
         "eg_launch_count": (C.c_longlong, [vp]),
         "eg_set_ilu_wait": (C.c_int, [vp, C.c_ulonglong, C.c_int]),
+        "eg_set_alloc_failure": (C.c_int, [vp, C.c_int]),
         "eg_check_pivot_reciprocal": (C.c_int, [_DP, _DP, C.c_longlong]),
         "eg_cell_norm_noalloc": (C.c_int, [C.POINTER(Desc), C.c_void_p, C.c_void_p, _DP]),
         "eg_create": (C.c_int, [C.POINTER(Desc), C.POINTER(Opts), C.POINTER(vp)]),
@@ -357,6 +358,10 @@ class Context:
     def set_ilu_wait(self, limit_ns: int = 0, starve: bool = False):
         """Test setting of the block ILU(0) device waits (eg_set_ilu_wait)."""
         self._check(self.lib.eg_set_ilu_wait(self.h, int(limit_ns), int(starve)))
+
+    def set_alloc_failure(self, nth: int = 0):
+        """Test setting of the device allocations (eg_set_alloc_failure)."""
+        self._check(self.lib.eg_set_alloc_failure(self.h, int(nth)))
 
     def pc_factor(self, factor: bool = True):
         self._check(self.lib.eg_pc_factor(self.h, int(factor)))

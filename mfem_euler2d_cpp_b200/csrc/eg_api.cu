@@ -55,7 +55,8 @@ static const char *kMessages[EG_ERR_COUNT] = {
 
 void *Ctx::alloc(size_t nbytes) {
   void *p = nullptr;
-  const cudaError_t e = cudaMalloc(&p, std::max<size_t>(nbytes, 16));
+  const bool refused = fail_alloc > 0 && --fail_alloc == 0;
+  const cudaError_t e = refused ? cudaErrorMemoryAllocation : cudaMalloc(&p, std::max<size_t>(nbytes, 16));
   if (e != cudaSuccess) {
     cudaGetLastError();
     fail(EG_ERR_OUT_OF_MEMORY, "device allocation of " + std::to_string(nbytes) + " bytes failed");
@@ -170,6 +171,16 @@ void Ctx::ensure_pc_hdg() {
   pc_hdg = alloc_n<double>((size_t)nf * t * t);
   piv_hdg = alloc_n<int>((size_t)nf * t);
 }
+
+// One size for the life of the context, whatever the first count is.
+void Ctx::ensure_work_cell(int cells) {
+  if (work_cell) return;
+  work_cell = alloc_n<double>((size_t)cells * m * m);
+  work_slots = cells;
+}
+// In front of the kernels that append: a list left by a call that failed before
+// it was read would be appended to, past its n entries.
+void Ctx::clear_redo() { EG_CUDA(cudaMemsetAsync(derr + 3, 0, sizeof(int), stream)); }
 
 static double now_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
@@ -1049,6 +1060,11 @@ int eg_set_ilu_wait(eg_ctx *ctx, unsigned long long limit_ns, int starve) {
       P.starve = ctx->c.ilu_starve;
     }
   });
+}
+
+int eg_set_alloc_failure(eg_ctx *ctx, int nth) {
+  if (!ctx || nth < 0) return EG_ERR_INVALID;
+  return guard(ctx, [&] { ctx->c.fail_alloc = nth; });
 }
 
 int eg_profile_enable(eg_ctx *ctx, int on) {

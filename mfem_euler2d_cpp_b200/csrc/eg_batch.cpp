@@ -170,6 +170,11 @@ long long estimate_bytes(const eg_request &r) {
   const long long q = r.k + 1, p = q * q, m = 4 * p, t = 4 * q, n = (long long)r.nx * r.ny, nf = 2 * n;
   const long long nu = n * m, nl = nf * t, N = std::max(nu, nl), R = 20;
   long long d = 14 * nu + 5 * nf * q + N * (R + 1) + 6 * N + 2 * nl;
+  // blocks m x m of the cells solved again by LU (a DG factor, or a condensation
+  // whose cell exceeds shared memory), one per SM at most
+  if (r.form == EG_FORM_DG || r.k >= 6) d += std::min(n, 148LL) * m * m;
+  // cell inverses of the clusters (k = 6: two CTAs each, 7: four, 8: six)
+  if (r.form == EG_FORM_HDG && r.k >= 6) d += std::min(n, 148LL / (2 * (r.k - 5))) * m * m;
   if (r.form == EG_FORM_HDG) {
     d += n * m * (4 * t + 1) + n * 4 * q * 17 + n * 4 * t + n * (q >= 5 ? 16 : 4) * t * t + 4 * nl + nf * t * t +
          nf * t / 2;

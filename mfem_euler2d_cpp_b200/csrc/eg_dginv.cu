@@ -154,6 +154,7 @@ void launch_inverse(Ctx &c, const double *u) {
 
 void launch_dg_inverse(Ctx &c, const double *u) {
   c.ensure_pc_dg();
+  c.clear_redo();
   {
     ProfScope ps(c, EG_K_DG_JACOBI, 1);
     switch (c.q) {  // shapes as in the condensation, which does the same inversion
@@ -171,16 +172,12 @@ void launch_dg_inverse(Ctx &c, const double *u) {
   const int count = c.herr[3];
   if (count == 0) return;
   ProfScope ps(c, EG_K_DG_JACOBI, 1);
-  const int grid = std::min(count, sm_count_dginv());
-  if (c.work_cell == nullptr || c.work_slots < grid) {
-    c.work_cell = c.alloc_n<double>((size_t)grid * c.m * c.m);
-    c.work_slots = grid;
-  }
+  c.ensure_work_cell(std::min(c.n, sm_count_dginv()));
+  const int grid = std::min(count, c.work_slots);
   EG_DISPATCH_Q(c.q, (dg_inverse_lu_kernel<Q><<<grid, 256, 0, c.stream>>>(
                          c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, c.pc_dg, c.work_cell, c.redo,
                          count, c.derr)));
   EG_CUDA(cudaGetLastError());
-  EG_CUDA(cudaMemsetAsync(c.derr + 3, 0, sizeof(int), c.stream));
   c.check_device_error();
 }
 

@@ -646,16 +646,11 @@ static void condense_redo(Ctx &c, const double *u, const double *r, int count) {
     constexpr size_t dyn = condense_dyn_bytes<Q>();
     auto kern = condense_kernel<Q>;
     if (dyn > 48 * 1024) EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    if (condense_mode<Q>() == 2 && (c.work_cell == nullptr || c.work_slots < grid)) {
-      constexpr int M = 4 * Q * Q;
-      c.work_cell = c.alloc_n<double>((size_t)grid * M * M);
-      c.work_slots = grid;
-    }
+    if (condense_mode<Q>() == 2) c.ensure_work_cell(std::min(c.n, sm_count_hdg()));
     kern<<<grid, 256, dyn, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, r, c.XY, c.Cb,
                                        c.sf, c.contrib, c.panels, c.work_cell, c.redo, count, c.derr);
   });
   EG_CUDA(cudaGetLastError());
-  EG_CUDA(cudaMemsetAsync(c.derr + 3, 0, sizeof(int), c.stream));
   launch_condensed_rhs(c);
 }
 
@@ -667,6 +662,7 @@ static void condense_redo(Ctx &c, const double *u, const double *r, int count) {
 // instead of 5 x 3: 2.16). From k = 6 on a cell takes a cluster.
 void condense_launch(Ctx &c, const double *u, const double *r) {
   c.ensure_hdg();
+  c.clear_redo();
   {
     ProfScope ps(c, EG_K_CONDENSE, 2);
     switch (c.q) {

@@ -171,6 +171,7 @@ struct Ctx {
   std::string err;
   long long bytes = 0;
   std::vector<void *> allocations;
+  int fail_alloc = 0;  // eg_set_alloc_failure
 
   // tables and metrics
   double *tab = nullptr;
@@ -192,9 +193,11 @@ struct Ctx {
   // which the Schur action then streams instead of X
   double *panels = nullptr;
   double *rhs = nullptr, *lam = nullptr, *tmp_trace = nullptr;  // nl
-  double *work_cell = nullptr;  // global LU workspace for large cells
+  double *work_cell = nullptr;  // LU of the cells solved again: work_slots blocks m x m (ensure_work_cell)
   int work_slots = 0;
-  int *redo = nullptr;          // n cells a condensation or DG factor solves again by pivoted LU (count in derr[3])
+  // up to n cells a condensation or DG factor solves again by pivoted LU; derr[3]
+  // counts them, and every launch that appends starts it from zero (clear_redo)
+  int *redo = nullptr;
   double *work_gj = nullptr;    // k >= 6 condensation: one m x m inverse per cluster
   int work_gj_slots = 0;
   // block Jacobi: explicit inverses (or, unfactored, the blocks), column-major:
@@ -266,6 +269,8 @@ struct Ctx {
   void ensure_krylov();
   void ensure_pc_dg();
   void ensure_pc_hdg();
+  void ensure_work_cell(int cells);  // for at most `cells` CTAs
+  void clear_redo();
   void sync();
   // one copy of the status words and scalars, and the stream synchronised
   void fetch_status();
