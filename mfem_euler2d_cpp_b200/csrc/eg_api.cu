@@ -136,40 +136,40 @@ void Ctx::raise_device_error() {
 }
 
 void Ctx::ensure_hdg() {
-  if (XY) return;
-  XY = alloc_n<double>((size_t)n * m * (4 * t + 1));
-  Cb = alloc_n<double>((size_t)n * 4 * q * 16);
-  sf = alloc_n<double>((size_t)n * 4 * q);
-  contrib = alloc_n<double>((size_t)n * 4 * t);
-  panels = alloc_n<double>((size_t)n * geo.npan * t * t);
-  if (!redo) redo = alloc_n<int>(n);
-  rhs = alloc_n<double>(nl);
-  lam = alloc_n<double>(nl);
-  tmp_trace = alloc_n<double>(nl);
+  if (tmp_trace) return;
+  need(XY, (size_t)n * m * (4 * t + 1));
+  need(Cb, (size_t)n * 4 * q * 16);
+  need(sf, (size_t)n * 4 * q);
+  need(contrib, (size_t)n * 4 * t);
+  need(panels, (size_t)n * geo.npan * t * t);
+  need(redo, n);
+  need(rhs, nl);
+  need(lam, nl);
+  need(tmp_trace, nl);
   EG_CUDA(cudaMemsetAsync(lam, 0, sizeof(double) * nl, stream));
 }
 
 void Ctx::ensure_krylov() {
-  if (V) return;
-  kN = std::max(nu, nl);
-  kR = opts.restart;
-  V = alloc_n<double>((size_t)kN * (kR + 1));
-  kw = alloc_n<double>(kN);
-  kz = alloc_n<double>(kN);
-  kres = alloc_n<double>(kN);
-  kcomb = alloc_n<double>(kN);
-  kcorr = alloc_n<double>(kN);
+  if (kcorr) return;
+  if (!V) {
+    kN = std::max(nu, nl);
+    kR = opts.restart;
+  }
+  need(V, (size_t)kN * (kR + 1));
+  need(kw, kN);
+  need(kz, kN);
+  need(kres, kN);
+  need(kcomb, kN);
+  need(kcorr, kN);
 }
 
 void Ctx::ensure_pc_dg() {
-  if (pc_dg) return;
-  pc_dg = alloc_n<double>((size_t)n * m * m);
-  if (!redo) redo = alloc_n<int>(n);
+  need(pc_dg, (size_t)n * m * m);
+  need(redo, n);
 }
 void Ctx::ensure_pc_hdg() {
-  if (pc_hdg) return;
-  pc_hdg = alloc_n<double>((size_t)nf * t * t);
-  piv_hdg = alloc_n<int>((size_t)nf * t);
+  need(pc_hdg, (size_t)nf * t * t);
+  need(piv_hdg, (size_t)nf * t);
 }
 
 // One size for the life of the context, whatever the first count is.
@@ -291,15 +291,21 @@ static void linear_solve(Ctx &c, int form, const double *rhs, double *x, double 
   // the element-assembled Schur entries come with the condensation
   const bool assembled = form == EG_FORM_DG ? c.opts.assembly != EG_ASSEMBLY_PARTIAL
                                             : c.opts.assembly == EG_ASSEMBLY_FULL;
+  const bool dense = c.opts.solver == EG_SOLVER_DENSE;
+  if (!refresh) {  // goes on with the preconditioner or factor of an earlier call
+    const bool there = dense ? c.dense_n == ops.N
+                       : c.opts.precond == EG_PC_BLOCK_ILU0 ? c.ilu[form].built
+                                                            : (form == EG_FORM_DG ? c.pc_dg : c.pc_hdg) != nullptr;
+    if (!there) fail(EG_ERR_INVALID, "no preconditioner built");
+  }
   double t0 = now_s();
   // DG partial assembly: PartialDGOperator::Refresh at the Newton state
   // (src/stepper.cpp:139), kept for the whole solve like the reference's
-  if (form == EG_FORM_DG && c.opts.assembly == EG_ASSEMBLY_PARTIAL && (refresh || !c.dgc_vol))
+  if (form == EG_FORM_DG && c.opts.assembly == EG_ASSEMBLY_PARTIAL && (refresh || !c.dgc_face))
     launch_dg_refresh(c, c.u);
   if (refresh && assembled) assemble_blocks(c, form);
   out.assembly = now_s() - t0;
   t0 = now_s();
-  const bool dense = c.opts.solver == EG_SOLVER_DENSE;
   if (refresh) {
     if (dense)
       dense_factor(c, form);  // src/linear.cpp:204-206 (no preconditioner)

@@ -573,7 +573,7 @@ static int sm_count();
 
 void launch_residual(Ctx &c, const double *u, const double *old, double *r) {
   ProfScope ps(c, EG_K_RESIDUAL, 2);
-  if (!c.dgc_h) c.dgc_h = c.alloc_n<double>((size_t)4 * c.nf * c.q);
+  c.need(c.dgc_h, (size_t)4 * c.nf * c.q);
   const int grid = (int)std::min<long long>(((long long)c.nf * c.q + 255) / 256, (long long)sm_count() * 16);
   EG_DISPATCH_Q(c.q, {
     using C = CellCfg<Q>;
@@ -586,10 +586,8 @@ void launch_residual(Ctx &c, const double *u, const double *old, double *r) {
 
 void launch_dg_refresh(Ctx &c, const double *u) {
   ProfScope ps(c, EG_K_DG_APPLY, 1);
-  if (!c.dgc_vol) {
-    c.dgc_vol = c.alloc_n<double>((size_t)32 * c.n * c.p);
-    c.dgc_face = c.alloc_n<double>((size_t)32 * c.nf * c.q);
-  }
+  c.need(c.dgc_vol, (size_t)32 * c.n * c.p);
+  c.need(c.dgc_face, (size_t)32 * c.nf * c.q);
   const int grid = sm_count() * 8;
   EG_DISPATCH_Q(c.q, {
     dg_refresh_volume_kernel<Q><<<grid, 256, 0, c.stream>>>(c.geo, c.tab, u, c.dgc_vol);
@@ -601,7 +599,7 @@ void launch_dg_refresh(Ctx &c, const double *u) {
 void launch_dg_apply_cached(Ctx &c, const double *x, double *y) {
   if (!c.dgc_vol) fail(EG_ERR_INVALID, "DG partial assembly used before its refresh");
   ProfScope ps(c, EG_K_DG_APPLY, 1);
-  if (!c.dgc_h) c.dgc_h = c.alloc_n<double>((size_t)4 * c.nf * c.q);
+  c.need(c.dgc_h, (size_t)4 * c.nf * c.q);
   const int grid = (int)std::min<long long>(((long long)c.nf * c.q + 255) / 256, (long long)sm_count() * 16);
   EG_DISPATCH_Q(c.q, {
     using C = CellCfg<Q>;

@@ -852,10 +852,8 @@ double launch_solve(Ctx &c, typename Op::Args &oa, SolveArgs<typename Op::Real> 
 template <class T>
 SolveArgs<T> solve_args(Ctx &c, const KrylovBufs<T> &kb, const T *rhs, T *x, double tol, int limit, bool zero_guess,
                         double rhs_norm, int N) {
-  if (!c.solve_bar) {
-    c.solve_bar = c.alloc_n<unsigned>(2);
-    c.solve_partials = c.alloc_n<double>((size_t)3 * (kGC + 1) * sm_count_gmres());
-  }
+  c.need(c.solve_bar, 2);
+  c.need(c.solve_partials, (size_t)3 * (kGC + 1) * sm_count_gmres());
   SolveArgs<T> s{};
   s.R = std::min(N, kb.R);
   s.limit = limit;
@@ -899,7 +897,7 @@ template <int Q>
 double solve_dg(Ctx &c, const KrylovBufs<double> &kb, const double *rhs, double *x, double tol, int limit,
                 bool zero_guess, double rhs_norm, int *count) {
   using Op = DgOp<Q>;
-  if (!c.dgc_h) c.dgc_h = c.alloc_n<double>((size_t)4 * c.nf * c.q);
+  c.need(c.dgc_h, (size_t)4 * c.nf * c.q);
   const int grid = solve_grid(c.n, 8. * c.n * ((double)c.m * c.m + 32 * c.p + 64 * c.q), c.nu);
   const int per = (c.n + grid - 1) / grid;
   // warps per cell of the block apply: the fewest whose last round of cells

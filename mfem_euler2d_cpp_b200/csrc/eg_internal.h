@@ -265,6 +265,13 @@ struct Ctx {
   T *alloc_n(size_t n) {
     return static_cast<T *>(alloc(n * sizeof(T)));
   }
+  // Allocates p unless it is there. A workspace of several arrays counts as
+  // there when its last one is: after a refused allocation the next call goes
+  // on where that one ended.
+  template <class T>
+  void need(T *&p, size_t n) {
+    if (!p) p = alloc_n<T>(n);
+  }
   void ensure_hdg();
   void ensure_krylov();
   void ensure_pc_dg();

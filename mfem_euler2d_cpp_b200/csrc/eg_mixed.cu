@@ -219,23 +219,23 @@ struct MixedHdgOps : LinearOpsT<float> {
 };
 
 void ensure_mixed(Ctx &c) {
-  if (c.Xf) return;
+  if (c.kfrhs) return;
   c.ensure_krylov();  // fixes the restart length both solvers use
   // FP32 copy of X, or of the 16 Schur panels per cell where the FP64 Schur
   // action streams those (all 16 panels kept per cell)
-  c.Xf = c.alloc_n<float>((size_t)c.n * (c.geo.npan == 16 ? 16 * c.t * c.t : c.m * 4 * c.t));
-  c.pcf = c.alloc_n<float>((size_t)c.nf * c.t * c.t);
-  c.Df = c.alloc_n<float>(c.nl);
-  c.contribf = c.alloc_n<float>((size_t)c.n * 4 * c.t);
+  c.need(c.Xf, (size_t)c.n * (c.geo.npan == 16 ? 16 * c.t * c.t : c.m * 4 * c.t));
+  c.need(c.pcf, (size_t)c.nf * c.t * c.t);
+  c.need(c.Df, c.nl);
+  c.need(c.contribf, (size_t)c.n * 4 * c.t);
   const size_t N = c.nl;
-  c.kfV = c.alloc_n<float>(N * (c.kR + 1));
-  c.kfw = c.alloc_n<float>(N);
-  c.kfz = c.alloc_n<float>(N);
-  c.kfres = c.alloc_n<float>(N);
-  c.kfcomb = c.alloc_n<float>(N);
-  c.kfcorr = c.alloc_n<float>(N);
-  c.kfx = c.alloc_n<float>(N);
-  c.kfrhs = c.alloc_n<float>(N);
+  c.need(c.kfV, N * (c.kR + 1));
+  c.need(c.kfw, N);
+  c.need(c.kfz, N);
+  c.need(c.kfres, N);
+  c.need(c.kfcomb, N);
+  c.need(c.kfcorr, N);
+  c.need(c.kfx, N);
+  c.need(c.kfrhs, N);
 }
 
 }  // namespace
