@@ -182,6 +182,8 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_kernel(SweepArgs a) {
         const bool local = owner == g;
         ok = local ? wait_local(dl, (unsigned)js + 1, a.abort, a.err, a.limit_ns)
                    : wait_progress(a.progress + owner, need(a.tag, js, a.starve), a.abort, a.err, a.limit_ns);
+        // lanes that give up and lanes that do not may not part before a warp barrier
+        ok = __all_sync(0xffffffffu, ok);
         if (ok) {
           __threadfence_block();
           const bool in_ring = local && slot - js <= a.ring - W;
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_small_kernel(SweepArgs a) {
       }
     }
     if (copy) {
-      if (!mbar_wait(&bars[warp], phase, kCopySpinLimit)) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars[warp], phase, kCopySpinLimit))) {
         give_up(a.abort, a.err);
         // let the copy land before the CTA can exit; if even the longer drain
         // bound runs out, the copy may still write this CTA's shared memory:
@@ -411,24 +413,24 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_small_kernel(SweepArgs a) {
         load_block(k < nst ? stage + (size_t)k * BB : a.data + (size_t)(e0 + k) * BB);
         product(vb + k * B, -1.);
       }
-    // the CTA's own rows, the ones finished first in front
+    // the CTA's own rows, the ones finished first in front; a lane whose wait
+    // gives up goes on with whatever the ring holds, so that the warp reaches
+    // its barriers together, and all leave behind the last row
 #pragma unroll
     for (int k0 = 0; k0 < kMaxDeps; ++k0) {
       const int k = BACK ? kMaxDeps - 1 - k0 : k0;
-      if (k < ne && (dep[k].x >> kOwnerShift) == g && ok) {
+      if (k < ne && (dep[k].x >> kOwnerShift) == g) {
         const int js = dep[k].x & kSlotMask;
         load_block(k < nst ? stage + (size_t)k * BB : a.data + (size_t)(e0 + k) * BB);
-        ok = wait_local(dl, (unsigned)js + 1, a.abort, a.err, a.limit_ns);
-        if (ok) {
-          __threadfence_block();
-          const double *v = ring + (size_t)(js & (a.ring - 1)) * B;
-          if (slot - js > a.ring - W) {  // gone from the ring
-            for (int r = lane; r < B; r += 32) vb[k * B + r] = __ldcg(a.out + (size_t)dep[k].y * B + r);
-            __syncwarp();
-            v = vb + k * B;
-          }
-          product(v, -1.);
+        ok = wait_local(dl, (unsigned)js + 1, a.abort, a.err, a.limit_ns) && ok;
+        __threadfence_block();
+        const double *v = ring + (size_t)(js & (a.ring - 1)) * B;
+        if (slot - js > a.ring - W) {  // gone from the ring
+          for (int r = lane; r < B; r += 32) vb[k * B + r] = __ldcg(a.out + (size_t)dep[k].y * B + r);
+          __syncwarp();
+          v = vb + k * B;
         }
+        product(v, -1.);
       }
     }
     ok = __all_sync(0xffffffffu, ok);
