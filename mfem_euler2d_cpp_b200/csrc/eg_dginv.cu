@@ -169,7 +169,7 @@ void launch_dg_inverse(Ctx &c, const double *u) {
     EG_CUDA(cudaGetLastError());
   }
   c.check_device_error();
-  const int count = c.herr[3];
+  const int count = c.redo_count();
   if (count == 0) return;
   ProfScope ps(c, EG_K_DG_JACOBI, 1);
   c.ensure_work_cell(std::min(c.n, sm_count_dginv()));

@@ -681,7 +681,7 @@ void condense_launch(Ctx &c, const double *u, const double *r) {
 }
 
 bool condense_finish(Ctx &c, const double *u, const double *r) {
-  const int count = c.herr[3];
+  const int count = c.redo_count();
   if (count == 0) {
     c.raise_device_error();
     return false;

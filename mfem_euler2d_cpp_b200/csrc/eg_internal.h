@@ -198,6 +198,7 @@ struct Ctx {
   // up to n cells a condensation or DG factor solves again by pivoted LU; derr[3]
   // counts them, and every launch that appends starts it from zero (clear_redo)
   int *redo = nullptr;
+  bool redo_open = false;  // derr[3] may be nonzero
   double *work_gj = nullptr;    // k >= 6 condensation: one m x m inverse per cluster
   int work_gj_slots = 0;
   // block Jacobi: explicit inverses (or, unfactored, the blocks), column-major:
@@ -278,6 +279,7 @@ struct Ctx {
   void ensure_pc_hdg();
   void ensure_work_cell(int cells);  // for at most `cells` CTAs
   void clear_redo();
+  int redo_count();  // of the status fetched behind those kernels
   void sync();
   // one copy of the status words and scalars, and the stream synchronised
   void fetch_status();
