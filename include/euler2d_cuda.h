@@ -264,7 +264,9 @@ int eg_newton_residual(eg_ctx *ctx, double *residual_norm);
 /* One accepted damped Newton update (src/stepper.cpp:129-228), DG or HDG per
  * the context's form: Jacobian / condensation, PC, GMRES, recovery and the
  * recovered-residual refinement loop, validation and line search, all on the
- * device. old_norm = CellNorm(stage base). */
+ * device. residual_norm = CellNorm(EG_SLOT_R), as eg_newton_residual returns it,
+ * old_norm = CellNorm(stage base): the validation and line-search criteria take
+ * them; the linear solve forms the norm of its right-hand side by itself. */
 int eg_newton_update(eg_ctx *ctx, double residual_norm, double old_norm, eg_update_stats *st);
 
 /* --------------------------------------------------------- diagnostics */

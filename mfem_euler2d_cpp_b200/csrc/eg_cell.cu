@@ -572,6 +572,7 @@ void launch_admissible(Ctx &c, const double *u) {
 static int sm_count();
 
 void launch_residual(Ctx &c, const double *u, const double *old, double *r) {
+  if (r == c.r) c.r_norm = -1.;
   ProfScope ps(c, EG_K_RESIDUAL, 2);
   c.need(c.dgc_h, (size_t)4 * c.nf * c.q);
   const int grid = (int)std::min<long long>(((long long)c.nf * c.q + 255) / 256, (long long)sm_count() * 16);

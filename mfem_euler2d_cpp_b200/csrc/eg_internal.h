@@ -254,6 +254,10 @@ struct Ctx {
         *kfcorr = nullptr, *kfx = nullptr, *kfrhs = nullptr;
 
   bool residual_ready = false;
+  // cell_norm(r) where the residual call has formed it; negative: unknown.
+  // Whatever writes r or the metric drops it (launch_residual, eg_upload,
+  // the exchange with the trial, upload_desc).
+  double r_norm = -1.;
   bool condensed = false;
   // set when an aborted sweep's bulk copy did not land within its bound: the
   // context's device memory can no longer be trusted; only eg_destroy works
@@ -367,6 +371,7 @@ void launch_axpby(Ctx &c, int N, double a, const double *x, double b, const doub
 void launch_copy(Ctx &c, int N, const double *x, double *out);
 void launch_fill(Ctx &c, int N, double v, double *out);
 double cell_norm(Ctx &c, const double *x);
+double residual_cell_norm(Ctx &c);  // of c.r, kept in c.r_norm
 // Weighted restarted GMRES (src/linear.cpp:76-157). Returns the true residual
 // norm; sets *count. Throws Failure on breakdown / limit / non-finite.
 // known_rhs_norm >= 0 is the caller's weighted norm of rhs (saves a reduction

@@ -437,6 +437,7 @@ double wnorm(Ctx &c, const double *x, int N, const double *mtab, int period) {
   return std::sqrt(c.hscal[DS_NORM]);
 }
 double cell_norm(Ctx &c, const double *x) { return wnorm(c, x, c.nu, c.mtab_dg, c.m); }
+double residual_cell_norm(Ctx &c) { return c.r_norm = cell_norm(c, c.r); }
 
 void launch_axpby(Ctx &c, int N, double a, const double *x, double b, const double *y, double *out) {
   ProfScope ps(c, EG_K_VECTOR, 1);

@@ -171,7 +171,7 @@ struct Stepper {
         EG_CUDA(cudaEventRecord(c.ev0, c.stream));
         c.update_timer_open = true;
         if (!c.residual_ready) launch_residual(c, c.u, c.old, c.r);
-        rn = cell_norm(c, c.r);
+        rn = residual_cell_norm(c);
         c.last_residual_s = wall_s() - t0;
       }
       const double rms = physical_scale * rn;
