@@ -127,7 +127,7 @@ struct SweepArgs {
   unsigned long long tag;
   unsigned long long limit_ns;  // bound of every wait
   int starve;        // test setting: waits on other CTAs can never be met
-  uint4 *slots;      // small blocks: the rows' values for other CTAs
+  ulonglong2 *slots;      // small blocks: the rows' values for other CTAs
   unsigned epoch;
 };
 
@@ -253,23 +253,22 @@ __global__ void __launch_bounds__(256, 1) ilu_sweep_kernel(SweepArgs a) {
   }
 }
 
-// A row's values for other CTAs travel as self-validating words: each 8-byte
-// half of a slot carries 32 bits of a value and the sweep's epoch, so a reader
+// A row's values for other CTAs travel as self-validating words: each 64-bit
+// word of a slot carries 32 bits of a value and the sweep's epoch, so a reader
 // polls the values themselves (one trip through L2) instead of a counter that
-// is released behind a fence and then the values (three).
-__device__ __forceinline__ void put_slot(uint4 *p, double v, unsigned ep) {
-  asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"((unsigned)__double2loint(v)),
-               "r"(ep), "r"((unsigned)__double2hiint(v)), "r"(ep)
+// is released behind a fence and then the values (three). The two words are the
+// elements of a 64-bit vector access: the memory model makes an element one
+// access and promises nothing for the vector, so each word carries the epoch.
+__device__ __forceinline__ void put_slot(ulonglong2 *p, double v, unsigned ep) {
+  const unsigned long long e = (unsigned long long)ep << 32, b = (unsigned long long)__double_as_longlong(v);
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(e | (b & 0xffffffffull)), "l"(e | (b >> 32))
                : "memory");
 }
-__device__ __forceinline__ bool get_slot(const uint4 *p, unsigned ep, double &v) {
-  unsigned lo, e0, hi, e1;
-  asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(lo), "=r"(e0), "=r"(hi), "=r"(e1)
-               : "l"(p)
-               : "memory");
-  v = __hiloint2double((int)hi, (int)lo);
-  return e0 == ep && e1 == ep;
+__device__ __forceinline__ bool get_slot(const ulonglong2 *p, unsigned ep, double &v) {
+  unsigned long long lo, hi;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+  v = __longlong_as_double((long long)((hi << 32) | (lo & 0xffffffffull)));
+  return (unsigned)(lo >> 32) == ep && (unsigned)(hi >> 32) == ep;
 }
 
 // The sweep for blocks of at most kStageMaxB (every HDG degree, DG up to k =
@@ -1136,7 +1135,7 @@ void build_plan(Ctx &c, int form) {
   P.dinv = c.alloc_n<double>((size_t)P.rows * BB);
   P.w = c.alloc_n<double>((size_t)P.rows * P.B);
   if (P.staged) {
-    const size_t bytes = sizeof(uint4) * (size_t)P.rows * P.B;
+    const size_t bytes = sizeof(ulonglong2) * (size_t)P.rows * P.B;
     P.slots = c.alloc(bytes);
     EG_CUDA(cudaMemsetAsync(P.slots, 0, bytes, c.stream));
   }
@@ -1178,7 +1177,7 @@ void sweep(Ctx &c, IluPlan &P, const double *in, double *out) {
   a.tag = (unsigned long long)(++P.epoch) << 32;
   a.limit_ns = P.wait_limit_ns;
   a.starve = P.starve;
-  a.slots = static_cast<uint4 *>(P.slots);
+  a.slots = static_cast<ulonglong2 *>(P.slots);
   a.epoch = P.epoch;
   if constexpr (S <= 2) {
     if (P.staged) {

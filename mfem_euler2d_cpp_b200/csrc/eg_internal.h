@@ -144,7 +144,7 @@ struct IluPlan {
   // while the preconditioner is block Jacobi, a separate array under ILU(0))
   double *asmd = nullptr, *asm_own = nullptr;
   double *work = nullptr;                        // factor slab for large blocks
-  void *slots = nullptr;                         // small blocks: rows of a sweep for other CTAs (uint4 per entry)
+  void *slots = nullptr;                         // small blocks: rows of a sweep for other CTAs (two 64-bit words per entry)
   unsigned long long *progress = nullptr;        // one counter per CTA of a sweep
   int *abort = nullptr;
   unsigned epoch = 0;
