@@ -24,6 +24,19 @@ void cuda_check(cudaError_t e, const char *what) {
   fail(EG_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+int device_sms() {
+  static const int n = [] {
+    int sms = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaGetLastError();
+      sms = 148;
+    }
+    return sms;
+  }();
+  return n;
+}
+
 static const char *kMessages[EG_ERR_COUNT] = {
     "ok",
     "invalid argument",

@@ -569,13 +569,11 @@ void launch_admissible(Ctx &c, const double *u) {
   EG_CUDA(cudaGetLastError());
 }
 
-static int sm_count();
-
 void launch_residual(Ctx &c, const double *u, const double *old, double *r) {
   if (r == c.r) c.r_norm = -1.;
   ProfScope ps(c, EG_K_RESIDUAL, 2);
   c.need(c.dgc_h, (size_t)4 * c.nf * c.q);
-  const int grid = (int)std::min<long long>(((long long)c.nf * c.q + 255) / 256, (long long)sm_count() * 16);
+  const int grid = (int)std::min<long long>(((long long)c.nf * c.q + 255) / 256, (long long)device_sms() * 16);
   EG_DISPATCH_Q(c.q, {
     using C = CellCfg<Q>;
     const int blocks = (c.n + C::CPB - 1) / C::CPB;
@@ -589,7 +587,7 @@ void launch_dg_refresh(Ctx &c, const double *u) {
   ProfScope ps(c, EG_K_DG_APPLY, 1);
   c.need(c.dgc_vol, (size_t)32 * c.n * c.p);
   c.need(c.dgc_face, (size_t)32 * c.nf * c.q);
-  const int grid = sm_count() * 8;
+  const int grid = device_sms() * 8;
   EG_DISPATCH_Q(c.q, {
     dg_refresh_volume_kernel<Q><<<grid, 256, 0, c.stream>>>(c.geo, c.tab, u, c.dgc_vol);
     dg_refresh_face_kernel<Q><<<grid, 256, 0, c.stream>>>(c.geo, c.tab, frozen_of(c), u, c.dgc_face);
@@ -601,7 +599,7 @@ void launch_dg_apply_cached(Ctx &c, const double *x, double *y) {
   if (!c.dgc_vol) fail(EG_ERR_INVALID, "DG partial assembly used before its refresh");
   ProfScope ps(c, EG_K_DG_APPLY, 1);
   c.need(c.dgc_h, (size_t)4 * c.nf * c.q);
-  const int grid = (int)std::min<long long>(((long long)c.nf * c.q + 255) / 256, (long long)sm_count() * 16);
+  const int grid = (int)std::min<long long>(((long long)c.nf * c.q + 255) / 256, (long long)device_sms() * 16);
   EG_DISPATCH_Q(c.q, {
     using C = CellCfg<Q>;
     const int blocks = (c.n + C::CPB - 1) / C::CPB;
@@ -622,21 +620,10 @@ void launch_dg_apply(Ctx &c, const double *u, const double *x, double *y) {
   EG_CUDA(cudaGetLastError());
 }
 
-static int sm_count() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 void launch_dg_jacobi(Ctx &c, const double *u) {
   c.ensure_pc_dg();
   ProfScope ps(c, EG_K_DG_JACOBI, 1);
-  const int grid = std::min(c.n, sm_count() * 8);
+  const int grid = std::min(c.n, device_sms() * 8);
   EG_DISPATCH_Q(c.q, dg_jacobi_kernel<Q><<<grid, 256, 0, c.stream>>>(c.geo, c.tab, frozen_of(c), u, c.pc_dg));
   EG_CUDA(cudaGetLastError());
 }

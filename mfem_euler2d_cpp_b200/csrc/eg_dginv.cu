@@ -128,24 +128,13 @@ __global__ void __launch_bounds__(256) block_inverse_cm_apply_kernel(const doubl
   }
 }
 
-int sm_count_dginv() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 template <int Q, int WR, int WC, int DED, int MINB>
 void launch_inverse(Ctx &c, const double *u) {
   using C = InvCfg<Q, WR, WC, DED>;
   constexpr size_t dyn = sizeof(double) * (size_t)C::REGION;
   auto kern = dg_inverse_kernel<Q, WR, WC, DED, MINB>;
   EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-  const int grid = std::min(c.n, sm_count_dginv() * MINB);
+  const int grid = std::min(c.n, device_sms() * MINB);
   kern<<<grid, C::THREADS, dyn, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, c.pc_dg,
                                             c.redo, c.derr + 3);
 }
@@ -172,7 +161,7 @@ void launch_dg_inverse(Ctx &c, const double *u) {
   const int count = c.redo_count();
   if (count == 0) return;
   ProfScope ps(c, EG_K_DG_JACOBI, 1);
-  c.ensure_work_cell(std::min(c.n, sm_count_dginv()));
+  c.ensure_work_cell(std::min(c.n, device_sms()));
   const int grid = std::min(count, c.work_slots);
   EG_DISPATCH_Q(c.q, (dg_inverse_lu_kernel<Q><<<grid, 256, 0, c.stream>>>(
                          c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, c.pc_dg, c.work_cell, c.redo,

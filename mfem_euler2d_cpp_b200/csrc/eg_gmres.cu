@@ -800,17 +800,6 @@ __global__ void __launch_bounds__(kGT, 1) gmres_kernel(typename Op::Args oa, Sol
   }
 }
 
-int sm_count_gmres() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 // CTAs of a solve over `cells` cells whose operator streams `bytes` per step on
 // vectors of N entries: one per 256 KB or 444 entries, at least 16, at most
 // one per SM, and no CTA with a nearly idle second round of cells. More CTAs
@@ -822,7 +811,7 @@ int sm_count_gmres() {
 // 148 CTAs each, 72 to 75 ms with 37 to 74.
 int solve_grid(int cells, double bytes, int N) {
   const double want = std::max(16., std::max(bytes / 262144., N / 444.));
-  const int cap = std::min(sm_count_gmres(), cells);
+  const int cap = std::min(device_sms(), cells);
   const int grid = std::max(1, (int)std::min<double>(cap, std::ceil(want)));
   int per = (cells + grid - 1) / grid;  // no more CTAs than the fullest ones need
   if (per > kGW && per < 2 * kGW && (cells + kGW - 1) / kGW <= cap) per = kGW;
@@ -853,7 +842,7 @@ template <class T>
 SolveArgs<T> solve_args(Ctx &c, const KrylovBufs<T> &kb, const T *rhs, T *x, double tol, int limit, bool zero_guess,
                         double rhs_norm, int N) {
   c.need(c.solve_bar, 2);
-  c.need(c.solve_partials, (size_t)3 * (kGC + 1) * sm_count_gmres());
+  c.need(c.solve_partials, (size_t)3 * (kGC + 1) * device_sms());
   SolveArgs<T> s{};
   s.R = std::min(N, kb.R);
   s.limit = limit;

@@ -608,24 +608,13 @@ __global__ void __launch_bounds__(256) block_gemv_kernel(const double *__restric
 }
 
 // ================================================================ launchers
-static int sm_count_hdg() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 template <int Q, int WR, int WC, int DED, int MINB>
 static void launch_condense_inv(Ctx &c, const double *u, const double *r) {
   using C = InvCfg<Q, WR, WC, DED>;
   constexpr size_t dyn = sizeof(double) * (size_t)(C::REGION + condense_inv_aux<Q, WR, WC>());
   auto kern = condense_inv_kernel<Q, WR, WC, DED, MINB>;
   EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-  const int grid = std::min(c.n, sm_count_hdg() * MINB);
+  const int grid = std::min(c.n, device_sms() * MINB);
   kern<<<grid, C::THREADS, dyn, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, r, c.XY, c.Cb,
                                             c.sf, c.contrib, c.panels, c.redo, c.derr + 3);
 }
@@ -641,12 +630,12 @@ static void launch_condensed_rhs(Ctx &c) {
 // partial pivoting; `count` of them in c.redo.
 static void condense_redo(Ctx &c, const double *u, const double *r, int count) {
   ProfScope ps(c, EG_K_CONDENSE, 2);
-  const int grid = std::min(count, sm_count_hdg());
+  const int grid = std::min(count, device_sms());
   EG_DISPATCH_Q(c.q, {
     constexpr size_t dyn = condense_dyn_bytes<Q>();
     auto kern = condense_kernel<Q>;
     if (dyn > 48 * 1024) EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    if (condense_mode<Q>() == 2) c.ensure_work_cell(std::min(c.n, sm_count_hdg()));
+    if (condense_mode<Q>() == 2) c.ensure_work_cell(std::min(c.n, device_sms()));
     kern<<<grid, 256, dyn, c.stream>>>(c.geo, c.tab, Frozen{c.fa, c.fbb, c.flw, c.frw, c.fpen}, u, r, c.XY, c.Cb,
                                        c.sf, c.contrib, c.panels, c.work_cell, c.redo, count, c.derr);
   });
@@ -701,7 +690,7 @@ void condense(Ctx &c, const double *u, const double *r) {
 
 void launch_schur_apply(Ctx &c, const double *v, double *y) {
   ProfScope ps(c, EG_K_SCHUR_APPLY, 2);
-  const int grid = std::min(c.n, sm_count_hdg() * 16);
+  const int grid = std::min(c.n, device_sms() * 16);
   if (c.geo.npan == 16) {
     switch (c.q) {
 #define EG_PG(QQ)                                                                                          \
@@ -727,7 +716,7 @@ void launch_schur_apply(Ctx &c, const double *v, double *y) {
 
 void launch_recover(Ctx &c, const double *lam, double *du) {
   ProfScope ps(c, EG_K_RECOVER, 1);
-  const int grid = std::min(c.n, sm_count_hdg() * 16);
+  const int grid = std::min(c.n, device_sms() * 16);
   EG_DISPATCH_Q(c.q, (cell_gemv_kernel<Q, true><<<grid, 128, 0, c.stream>>>(c.geo, c.tab, c.XY, c.Cb,
                                                                            lam, du, nullptr)));
   EG_CUDA(cudaGetLastError());
@@ -761,8 +750,8 @@ void launch_block_inverse_apply(Ctx &c, const double *inv, int nblocks, int bs, 
 void launch_schur_jacobi(Ctx &c, bool factor) {
   c.ensure_pc_hdg();
   ProfScope ps(c, EG_K_SCHUR_JACOBI, 1);
-  const int grid = std::min(c.nf, sm_count_hdg() * 32);
-  const int wgrid = std::min((c.nf + 3) / 4, sm_count_hdg() * 32);  // 4 warps (faces) per CTA
+  const int grid = std::min(c.nf, device_sms() * 32);
+  const int wgrid = std::min((c.nf + 3) / 4, device_sms() * 32);  // 4 warps (faces) per CTA
   switch (c.t) {
 #define EG_SJW(TT)                                                                                     \
   case TT:                                                                                             \

@@ -866,17 +866,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-int sm_count_ilu() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 // ------------------------------------------------------------ host: plan
 template <class Kern>
 int per_sm(Kern kern, int block, size_t smem) {
@@ -1048,7 +1037,7 @@ void build_plan(Ctx &c, int form) {
   }
   if (P.maxl > kMaxDeps || P.maxu > kMaxDeps) fail(EG_ERR_INVALID, "block ILU row too long");
   // launch shapes; every CTA of a sweep must be resident (cooperative launch)
-  const int sms = sm_count_ilu();
+  const int sms = device_sms();
   const size_t BB = (size_t)P.B * P.B;
   const int S = (P.B + 31) / 32;
   P.staged = P.B <= kStageMaxB ? 1 : 0;
@@ -1264,7 +1253,7 @@ void factor_dispatch(Ctx &c, IluPlan &P) {
 // Numeric blocks of the plan's structure into dst (nnzb x B^2, column-major).
 void fill_blocks(Ctx &c, int form, IluPlan &P, double *dst) {
   const bool hdg = form == EG_FORM_HDG;
-  const int sms = sm_count_ilu();
+  const int sms = device_sms();
   if (hdg) {
     const double *pan16 = c.geo.npan == 16 ? c.panels : P.panels16;
     if (c.geo.npan != 16) {

@@ -34,6 +34,8 @@ struct Failure {
 [[noreturn]] void fail(int status, const std::string &msg);
 void cuda_check(cudaError_t e, const char *what);
 #define EG_CUDA(call) ::eg::cuda_check((call), #call)
+// SMs of the device, asked once (by one of the threads that call it first).
+int device_sms();
 
 // Fixed grid of the deterministic reductions (partials are summed in block
 // order by the last block to finish).

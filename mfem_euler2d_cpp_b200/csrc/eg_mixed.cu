@@ -152,17 +152,6 @@ __global__ void __launch_bounds__(256)
   x[id] = acc;
 }
 
-int sm_count_mixed() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 // Inner operators: FP32 Schur action and FP32 block-Jacobi apply.
 struct MixedHdgOps : LinearOpsT<float> {
   explicit MixedHdgOps(Ctx &c) {
@@ -173,7 +162,7 @@ struct MixedHdgOps : LinearOpsT<float> {
   }
   void apply(Ctx &c, const float *x, float *y) override {
     ProfScope ps(c, EG_K_SCHUR_APPLY, 2);
-    const int grid = std::min(c.n, sm_count_mixed() * 16);
+    const int grid = std::min(c.n, device_sms() * 16);
     if (c.geo.npan == 16) {  // Xf holds the FP32 panels
       switch (c.q) {
 #define EG_PGF(QQ)                                                                                    \
