@@ -869,8 +869,17 @@ __global__ void __launch_bounds__(256)
 // ------------------------------------------------------------ host: plan
 template <class Kern>
 int per_sm(Kern kern, int block, size_t smem) {
-  // the opt-in covers dynamic sizes whose sum with the static shared memory passes 48 KB
-  if (smem > 0) EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // The opt-in is the most the kernel can have, not smem: it belongs to the
+  // function, and the sizes differ between meshes (a factor row has more updates
+  // on 3 x 3 cells than on 12 x 10), so one context would lower another's.
+  if (smem > 0) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa{};
+    EG_CUDA(cudaGetDevice(&dev));
+    EG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    EG_CUDA(cudaFuncGetAttributes(&fa, kern));
+    EG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+  }
   int n = 0;
   EG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, smem));
   return n;
