@@ -452,8 +452,9 @@ long long eg_launch_count(const eg_ctx *ctx);
 int eg_check_pivot_reciprocal(const double *x, double *y, long long n);
 
 /* Test setting of the device waits (no reference counterpart: the reference
- * is serial). limit_ns bounds every wait of the block ILU(0) factor and sweeps
- * and of the one-launch GMRES solve (0 restores the default, 250 ms); starve != 0
+ * is serial). limit_ns bounds the waits of the block ILU(0) factor and sweeps
+ * (the time in which no row of the launch is finished; noticed within twice
+ * that) and of the one-launch GMRES solve (0 restores the default, 250 ms); starve != 0
  * makes every wait on another CTA unreachable, so that the next factor or
  * apply runs out its bound, returns EG_ERR_WAIT_LIMIT and leaves the context
  * usable. Applies to both forms' plans, including ones built later. */

@@ -125,10 +125,13 @@ constexpr int kArnoldiGroup = 4;
 // doubles) instead of X (m x 4t): fewer bytes from q = 5 (k = 4) on.
 __host__ __device__ constexpr bool schur_panels_full(int q) { return q >= 5; }
 
-// Bound of a device-side wait of the block ILU(0) factor and sweeps. The
-// longest legitimate wait is bounded by one whole factor or sweep (45 ms for
-// the factor at 128 x 128 Q4 HDG); 250 ms leaves a wide margin and still ends
-// a wait on a row that never comes within a fraction of a second.
+// Bound of the device-side waits. Block ILU(0) factor and sweeps: the time in
+// which no row of the launch is finished (a row of the largest block, 324,
+// takes up to 70 ms in the factor, 16 rows of the sweeps far less). One-launch
+// GMRES: a barrier, which lasts a part of a Krylov step (30 ms when it streams
+// all of the device's memory). Neither counts time before the launch: a
+// cooperative launch starts with all of its CTAs or with none. 250 ms leaves a
+// margin and still ends a wait that nothing will meet within a second.
 constexpr unsigned long long kIluWaitLimitNs = 250ull * 1000 * 1000;
 
 // Block ILU(0) of one form (FixedBlockILU, src/block_ilu.cpp:10-109): fixed
@@ -150,8 +153,8 @@ struct IluPlan {
   unsigned long long *progress = nullptr;        // one counter per CTA of a sweep
   int *abort = nullptr;
   unsigned epoch = 0;
-  // bound of every device-side wait of the factor and the sweeps; starve (a
-  // test setting) makes every wait on another CTA unreachable
+  // bound of the device-side waits of the factor and the sweeps; starve (a test
+  // setting) makes every wait on another CTA unreachable
   unsigned long long wait_limit_ns = kIluWaitLimitNs;
   int starve = 0;
   int grid_factor = 0, grid_sweep = 0, sweep_warps = 0, staged = 0, ring = 0, maxrow = 0, maxupd = 0;
