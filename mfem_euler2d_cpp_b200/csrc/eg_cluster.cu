@@ -494,9 +494,11 @@ void dg_launch(Ctx &c, const double *u) {
 
 }  // namespace
 
-// Shapes: the fewest CTAs whose registers hold the matrix without spills (k = 6:
-// 35 tiles for each of 10 warps and one more for the pivot blocks; k = 7: 16
-// for 16; k = 8: 28 for 12). Clusters of 2 fill all 148 SMs, of 4 and 6 132.
+// Shapes: the fewest CTAs whose registers hold the tiles (k = 6: 35 tiles for
+// each of 10 warps and one more for the pivot blocks; k = 7: 16 for 16; k = 8:
+// 28 for 12). What a panel needs besides is spilled in part: 518 bytes stored
+// and 1416 loaded at k = 6 (140 of 168 registers are tiles), 48 and 216 at k =
+// 7, 116 and 688 at k = 8. Clusters of 2 fill all 148 SMs, of 4 and 6 132.
 // Condensation with a warp for the pivot blocks against tile warps in turn:
 // 8.10 against 9.12 ms at k = 6 (64x64 cells), but 5.21 against 4.74 at k = 7
 // and 13.3 against 11.8 at k = 8 (32x32), where it costs the others registers.

@@ -301,7 +301,7 @@ __device__ __forceinline__ bool get_slot(const ulonglong2 *p, unsigned ep, doubl
 // A row's products are four partial sums each, unrolled; its neighbours' rows
 // in other CTAs are polled together and folded in before its own CTA's.
 // 48x48 Q4, forward and backward sweep: 1190 us with the counters and run-time
-// block sizes of the kernel above, 417 here.
+// block sizes of the kernel above, 404 here.
 template <int B, bool BACK>
 __global__ void __launch_bounds__(256, 1) ilu_sweep_small_kernel(SweepArgs a) {
   constexpr int S = (B + 31) / 32, BB = B * B;
